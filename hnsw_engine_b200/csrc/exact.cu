@@ -11,9 +11,10 @@
 //     normalised rows); every (query, row) with a <= tau_q + margin_q is appended to the query's
 //     candidate list. margin_q = 2 e_q where e_q bounds |a - exact| for this arithmetic, so every true
 //     top-k row survives whenever tau_q is at least the k-th smallest approximate distance.
-//  3. tau_q: pass one runs the filter on a prefix of the data with tau = +inf, and a radix select
-//     takes the k-th smallest approximate distance of that prefix (an upper bound of the global one).
-//     Pass two filters all rows; a second select tightens tau to the k-th smallest candidate.
+//  3. tau_q: pass one runs the filter on a sample of the data's tiles with tau = +inf, and a radix
+//     select takes a low rank of its approximate distances (sample_rank): all but surely at or above
+//     the k-th smallest of all rows, which pass two checks. Pass two filters all rows; a second
+//     select tightens tau to the k-th smallest candidate.
 //  4. rerank: float64 distances (sequential over dimensions) of the surviving candidates, best k by
 //     (distance, id) -- ties to the lower id, as np.lexsort((ids, exact)) in the reference.
 // Waits on mbarriers are bounded by a wall-clock limit; on expiry the kernel records an error,
@@ -42,26 +43,19 @@ namespace hbx {
 constexpr int BM = 128;  // queries per tile (TMEM lanes)
 constexpr int BN = 256;  // data rows per tile (TMEM columns per accumulator)
 constexpr int BK = 64;   // K elements per stage (128 bytes of BF16: one swizzle-128B row)
-constexpr int STAGES = 4;
+constexpr int MAX_STAGES = 6;
 constexpr int A_BYTES = BM * BK * 2;
 constexpr int B_BYTES = BN * BK * 2;
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-// Epilogue warps: EPI_WARPS / 4 per TMEM lane quarter, taking a tile's CW-column chunks in turn.
-// Narrower chunks need fewer registers per thread, which leaves room for more epilogue warps to
-// hide the TMEM-load and arithmetic latencies.
-#ifndef HB_EPI_WARPS
-#define HB_EPI_WARPS 20
-#endif
-#ifndef HB_EPI_CW
-#define HB_EPI_CW 16
-#endif
-constexpr int EPI_WARPS = HB_EPI_WARPS;
-constexpr int CW = HB_EPI_CW;  // columns per TMEM load (16 or 32)
-static_assert(CW == 16 || CW == 32, "chunks of 16 or 32 columns");
-constexpr int EPI_PER_QUARTER = EPI_WARPS / 4;
+// Epilogue warps: EPI_PER_QUARTER per TMEM lane quarter; each takes the two CW-column chunks
+// part and part + EPI_PER_QUARTER of a tile, so every warp has the same work in every tile.
+constexpr int EPI_PER_QUARTER = 4;
+constexpr int EPI_WARPS = 4 * EPI_PER_QUARTER;
+constexpr int CW = 32;  // columns per TMEM load
+static_assert(BN == 2 * CW * EPI_PER_QUARTER, "two chunks a warp and tile");
 constexpr int FILTER_THREADS = 128 + 32 * EPI_WARPS;
-constexpr int BAR_BYTES = 256;  // barriers and flags after the stage buffers and the |x|^2 ring
+constexpr int BAR_BYTES = 512;  // barriers and flags after the operand buffers and the |x|^2 ring
 constexpr int XSLOTS = 4;       // |x|^2 ring slots (one tile's BN values each)
+constexpr int SMEM_MAX = 227 * 1024;
 // Rows of at least COOP_DIM dimensions are re-scored by the whole warp, one candidate at a time.
 constexpr int COOP_DIM = 256;
 // Byte rows: one result in VERIFY_EVERY of each query is re-scored in float64 as a check.
@@ -86,16 +80,19 @@ constexpr int32_t I8_PAD = 0x3fffffff;
 
 struct FilterParams {
     int32_t nq;            // valid queries
-    int32_t row_begin;     // first data row of this pass
-    int32_t row_end;       // one past the last data row of this pass
+    int32_t row_end;       // one past the last data row
+    int32_t tiles;         // tiles of BN rows in this pass: 0, tile_stride, 2 tile_stride, ...
+    int32_t tile_stride;
     int32_t kchunks;       // K' / BK
+    int32_t stages;        // operand stages in flight
+    int32_t a_resident;    // the query tile's operand is loaded once and stays (else with each stage)
     int32_t tiles_per_split;
     int32_t metric;
     const float *qq;       // |q|^2 per query (l2)
-    const float *xx;       // |x|^2 per row (l2)
+    const float *xx;       // per row: |x|^2 (l2) or 0; +inf past the data rows
     const int32_t *qqi;    // byte rows: exact |q|^2 per query (l2)
-    const int32_t *xxi;    // byte rows: exact |x|^2 per row (l2)
-    const float *thr;      // per query: tau + margin (+inf in pass one)
+    const int32_t *xxi;    // byte rows: exact |x|^2 (l2) or 0; I8_PAD past the data rows
+    const float *thr;      // per query: tau + margin (NULL: +inf, the threshold pass)
     // Candidates in segments: every epilogue thread of the grid owns one segment of its query's
     // list (segment = row split x epilogue part), so appends need no atomics. Segment s of query q
     // starts at (q * nseg + s) * cap.
@@ -103,7 +100,7 @@ struct FilterParams {
     int32_t *cand_id;      // (nq, nseg, cap) row ids
     int32_t *cand_cnt;     // (nq, nseg) appended counts (may exceed cap: overflow)
     int32_t cap;           // entries per segment
-    int32_t block_min;     // 1: append only the minimum of each (tile, part) block (threshold pass)
+    int32_t mul;           // -2 (l2) or -1 (see EpiThread)
     int32_t *err;          // nonzero: a bounded wait expired
 };
 
@@ -218,8 +215,9 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
                  : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-    uint32_t r[32];
+// Issue a load of 32 accumulator columns; tmem_wait makes the registers readable (they are its
+// operands, so no use of them can be moved before the wait).
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[CW]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
         "%12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, "
@@ -230,62 +228,144 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
           "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
           "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
-        "%12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[CW]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]),
+                   "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]),
+                   "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]),
+                   "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
+                   "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27])
+                 :
+                 : "memory");
+    asm volatile("" : "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31]) : : "memory");
 }
 
-template <int W>
-__device__ __forceinline__ void tmem_ld(uint32_t taddr, float (&v)[W]) {
-    if constexpr (W == 16) tmem_ld16(taddr, v);
-    else tmem_ld32(taddr, v);
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]) : : "memory");
 }
 
-// I8: byte rows on kind::i8 (exact integer filter values); otherwise BF16 terms on kind::f16.
+__device__ __forceinline__ int32_t min3(int32_t a, int32_t b, int32_t c) { return __vimin3_s32(a, b, c); }
+__device__ __forceinline__ float min3(float a, float b, float c) { return fminf(fminf(a, b), c); }
+__device__ __forceinline__ int32_t min2(int32_t a, int32_t b) { return min(a, b); }
+__device__ __forceinline__ float min2(float a, float b) { return fminf(a, b); }
+
+// What one epilogue thread (one query of the tile) carries through its chunks. A row's filter value is
+// a = v + add with v = |x|^2 - 2 q.x (l2) or -q.x.
 template <bool I8>
+struct EpiThread {
+    using V = std::conditional_t<I8, int32_t, float>;
+    V add;       // |q|^2 (l2), 0 (ip), 1 (cosine)
+    V thr;       // a candidate has v <= thr (byte path) or fl(v + add) <= thr (BF16 path)
+    V mul;       // -2 (l2) or -1, from a kernel argument: on bytes that keeps the multiply-add on the FMA
+                 // pipe (of a constant the compiler makes shifts and adds, on the pipe of the minima)
+    float *cv;
+    int32_t *ci;
+    int cnt, cap;
+
+    // x: the row's term from the ring: |x|^2 (l2) or 0; above every threshold past the data rows
+    __device__ __forceinline__ V value(uint32_t r, uint32_t x) const {
+        if constexpr (I8) return int32_t(r) * mul + int32_t(x);
+        else return fmaf(mul, __uint_as_float(r), __uint_as_float(x));
+    }
+    __device__ __forceinline__ bool pass(V v) const {
+        if constexpr (I8) return v <= thr;
+        else return v + add <= thr;
+    }
+
+    // Minima of the groups of four of a chunk of CW accumulators, and of the chunk. xs: the terms of the
+    // chunk's rows in shared memory (the same addresses in every lane).
+    __device__ __forceinline__ V minima(const uint32_t (&r)[CW], const unsigned char *xs,
+                                        V (&mg)[CW / 4]) const {
+#pragma unroll
+        for (int g = 0; g < CW / 4; g++) {
+            const uint4 x = reinterpret_cast<const uint4 *>(xs)[g];
+            mg[g] = min2(min3(value(r[4 * g], x.x), value(r[4 * g + 1], x.y), value(r[4 * g + 2], x.z)),
+                         value(r[4 * g + 3], x.w));
+        }
+        return min3(min3(min3(mg[0], mg[1], mg[2]), mg[3], mg[4]), min2(mg[5], mg[6]), mg[7]);
+    }
+
+    // Appends the chunk's candidates: of the groups of four that hold one for some query of the warp,
+    // read again from TMEM (a loop of little code: unrolled over the chunk's registers, 16 diverging
+    // warps ran out of the instruction cache and the pass took twice the time). Every lane calls it.
+    __device__ __forceinline__ void append(uint32_t taddr, const unsigned char *xs, int col0, int valid,
+                                           const V (&mg)[CW / 4]) {
+        uint32_t gm = 0;
+#pragma unroll
+        for (int g = 0; g < CW / 4; g++) gm |= pass(mg[g]) ? 1u << g : 0u;
+        gm = __reduce_or_sync(0xffffffffu, gm);
+#pragma unroll 1
+        for (; gm; gm &= gm - 1) {
+            const int g = __ffs(gm) - 1;
+            uint32_t r[4];
+            tmem_ld4(taddr + uint32_t(4 * g), r);
+            const uint4 x = reinterpret_cast<const uint4 *>(xs)[g];
+            const V v[4] = {value(r[0], x.x), value(r[1], x.y), value(r[2], x.z), value(r[3], x.w)};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (pass(v[j]) && 4 * g + j < valid) {
+                    if (cnt < cap) {
+                        cv[cnt] = float(v[j] + add);
+                        ci[cnt] = col0 + 4 * g + j;
+                    }
+                    cnt++;
+                }
+            }
+        }
+    }
+};
+
+// The filter pass. What bounds it is the epilogue: a tile is 128 queries x 256 rows, its MMAs take 512
+// cycles of the tensor pipe on bytes at d = 128, and its 32,768 values go through 16 epilogue warps
+// in about 1,900 (issue slots 55% busy; 118 instructions a chunk of 32 columns and, where it holds a
+// candidate, about 60 more). So a warp takes exactly two chunks of a tile and loads the second while it
+// works on the first, a value costs one multiply-add (on the FMA pipe) and at most one minimum, rows past
+// the data carry a term above every threshold instead of a test on each value, and candidates are looked
+// for by groups of four in a small loop. The query tile's operand stays in shared memory over a
+// CTA's tiles wherever three stages of rows fit beside it (up to seven 128-byte chunks of K), else it
+// comes again with every tile. 10K queries x 1M x 128 bytes, both passes: 5.68 -> 2.60 ms; 1,000
+// x 200K x 100 floats: 177 -> 145 us.
+// I8: byte rows on kind::i8 (exact integer filter values); otherwise BF16 terms on kind::f16.
+// BMIN: the threshold pass over the sample, which keeps block minima only.
+template <bool I8, bool BMIN>
 __global__ void __launch_bounds__(FILTER_THREADS, 1)
     knn_filter_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const FilterParams p) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    // 1024-byte aligned stage buffers (swizzle-128B atoms), barriers after them.
+    // 1024-byte aligned operand buffers (swizzle-128B atoms): the resident query operand, the stages;
+    // then |x|^2 of a tile's BN rows (float or int32, 4 bytes each) in a ring of XSLOTS (the
+    // producer fills slot lt % XSLOTS, the epilogue reads it and releases it); then the barriers.
     unsigned char *smem = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    // |x|^2 of a tile's BN rows (float or int32, 4 bytes each) in a ring of XSLOTS, after the
-    // stages: the producer fills slot lt % XSLOTS, the epilogue reads it and releases it.
-    unsigned char *xring = smem + STAGES * STAGE_BYTES;
+    const int nst = p.stages;
+    const int a_bytes = p.a_resident ? p.kchunks * A_BYTES : 0;
+    const int stage_bytes = p.a_resident ? B_BYTES : A_BYTES + B_BYTES;
+    unsigned char *stages = smem + a_bytes;
+    unsigned char *xring = stages + nst * stage_bytes;
     uint64_t *full = reinterpret_cast<uint64_t *>(xring + XSLOTS * BN * 4);
-    uint64_t *empty = full + STAGES;
-    uint64_t *tfull = empty + STAGES;
+    uint64_t *empty = full + MAX_STAGES;
+    uint64_t *tfull = empty + MAX_STAGES;
     uint64_t *tempty = tfull + 2;
     uint64_t *xfull = tempty + 2;
     uint64_t *xempty = xfull + XSLOTS;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(xempty + XSLOTS);
+    uint64_t *afull = xempty + XSLOTS;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(afull + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int qt = blockIdx.x;
-    const int total_tiles = (p.row_end - p.row_begin + BN - 1) / BN;
     const int t0 = blockIdx.y * p.tiles_per_split;
-    const int t1 = min(total_tiles, t0 + p.tiles_per_split);
+    const int t1 = min(p.tiles, t0 + p.tiles_per_split);
     const int ntiles = max(0, t1 - t0);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; s++) {
+        for (int s = 0; s < nst; s++) {
             mbar_init(full + s, 1);
             mbar_init(empty + s, 1);
         }
@@ -297,6 +377,7 @@ __global__ void __launch_bounds__(FILTER_THREADS, 1)
             mbar_init(xfull + x, 1);
             mbar_init(xempty + x, EPI_WARPS);
         }
+        mbar_init(afull, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -316,8 +397,16 @@ __global__ void __launch_bounds__(FILTER_THREADS, 1)
         // ---------------------------------------------------------------- TMA producer
         int it = 0, xs = 0;  // stages and |x|^2 slots issued
         bool ok = true;
+        const bool a_once = p.a_resident && ntiles > 0;
+        if (a_once) {
+            mbar_expect_tx(afull, uint32_t(p.kchunks) * A_BYTES);
+            for (int kc = 0; kc < p.kchunks; kc++)
+                tma_load_2d(&tmA, afull, smem + kc * A_BYTES, kc * (I8 ? BK8 : BK), qt * BM);
+        }
+        int s = 0;
+        uint32_t par = 1;  // of the stage's release
         for (int lt = 0; lt < ntiles && ok; lt++) {
-            const int row0 = p.row_begin + (t0 + lt) * BN;
+            const int row0 = (t0 + lt) * p.tile_stride * BN;
             {  // the tile's |x|^2 (rows row0 .. row0 + BN - 1 < n_pad) into its ring slot
                 const int x = lt % XSLOTS;
                 if (!mbar_wait(xempty + x, ((lt / XSLOTS) & 1) ^ 1, abort_flag)) {
@@ -331,43 +420,41 @@ __global__ void __launch_bounds__(FILTER_THREADS, 1)
                 xs++;
             }
             for (int kc = 0; kc < p.kchunks; kc++, it++) {
-                const int s = it % STAGES;
-                const uint32_t par = ((it / STAGES) & 1) ^ 1;
                 if (!mbar_wait(empty + s, par, abort_flag)) {
                     ok = false;
                     break;
                 }
-                unsigned char *a = smem + s * STAGE_BYTES;
-                unsigned char *b = a + A_BYTES;
-                mbar_expect_tx(full + s, STAGE_BYTES);
-                tma_load_2d(&tmA, full + s, a, kc * (I8 ? BK8 : BK), qt * BM);
+                unsigned char *b = stages + s * stage_bytes;
+                mbar_expect_tx(full + s, uint32_t(stage_bytes));
                 tma_load_2d(&tmB, full + s, b, kc * (I8 ? BK8 : BK), row0);
+                if (!p.a_resident)
+                    tma_load_2d(&tmA, full + s, b + B_BYTES, kc * (I8 ? BK8 : BK), qt * BM);
+                if (++s == nst) {
+                    s = 0;
+                    par ^= 1;
+                }
             }
         }
         if (!ok) {
             atomicExch(p.err, 1);
             *abort_flag = 1;
         }
-        // Drain: every stage and |x|^2 slot issued must land before the CTA may exit.
-        const int issued = it;
-        for (int j = max(0, issued - STAGES); j < issued; j++) {
-            const int s = j % STAGES;
-            const uint32_t par = (j / STAGES) & 1;
+        // Drain: everything issued must land before the CTA may exit.
+        auto drain = [&](uint64_t *bar, uint32_t parity) {
             const unsigned long long t = now_ns();
-            while (!mbar_try(full + s, par) && now_ns() - t < WAIT_LIMIT_NS) {
+            while (!mbar_try(bar, parity) && now_ns() - t < WAIT_LIMIT_NS) {
             }
-        }
-        for (int j = max(0, xs - XSLOTS); j < xs; j++) {
-            const int x = j % XSLOTS;
-            const uint32_t par = (j / XSLOTS) & 1;
-            const unsigned long long t = now_ns();
-            while (!mbar_try(xfull + x, par) && now_ns() - t < WAIT_LIMIT_NS) {
-            }
-        }
+        };
+        for (int j = max(0, it - nst); j < it; j++) drain(full + j % nst, (j / nst) & 1);
+        for (int j = max(0, xs - XSLOTS); j < xs; j++) drain(xfull + j % XSLOTS, (j / XSLOTS) & 1);
+        if (a_once) drain(afull, 0);
     } else if (warp == 1 && lane == 0) {
         // ---------------------------------------------------------------- MMA issuer
         int it = 0;
         bool ok = true;
+        if (p.a_resident && ntiles > 0) ok = mbar_wait(afull, 0, abort_flag);
+        int s = 0, last = 0;
+        uint32_t par = 0, last_par = 0;
         for (int lt = 0; lt < ntiles && ok; lt++) {
             const int b = lt & 1;
             if (!mbar_wait(tempty + b, ((lt >> 1) & 1) ^ 1, abort_flag)) {
@@ -377,14 +464,13 @@ __global__ void __launch_bounds__(FILTER_THREADS, 1)
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t tmem_d = tmem_base + uint32_t(b * BN);
             for (int kc = 0; kc < p.kchunks; kc++, it++) {
-                const int s = it % STAGES;
-                if (!mbar_wait(full + s, (it / STAGES) & 1, abort_flag)) {
+                if (!mbar_wait(full + s, par, abort_flag)) {
                     ok = false;
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t a_addr = smem_u32(smem + s * STAGE_BYTES);
-                const uint32_t b_addr = a_addr + A_BYTES;
+                const uint32_t b_addr = smem_u32(stages + s * stage_bytes);
+                const uint32_t a_addr = p.a_resident ? smem_u32(smem + kc * A_BYTES) : b_addr + B_BYTES;
 #pragma unroll
                 for (int j = 0; j < 4; j++) {  // 32 bytes of K per instruction (16 BF16 or 32 bytes)
                     if constexpr (I8)
@@ -395,6 +481,12 @@ __global__ void __launch_bounds__(FILTER_THREADS, 1)
                                   (kc | j) != 0);
                 }
                 umma_commit(empty + s);
+                last = s;
+                last_par = par;
+                if (++s == nst) {
+                    s = 0;
+                    par ^= 1;
+                }
             }
             if (ok) umma_commit(tfull + b);
         }
@@ -402,45 +494,54 @@ __global__ void __launch_bounds__(FILTER_THREADS, 1)
             atomicExch(p.err, 1);
             *abort_flag = 1;
         }
-        // Every MMA issued must finish before TMEM is released: commit one more arrival on a
-        // stage barrier and wait for it (tcgen05.commit tracks all prior MMAs of this thread).
+        // Every MMA issued must finish before TMEM is released: wait for the last stage's commit
+        // (tcgen05.commit tracks all prior MMAs of this thread).
         if (it > 0) {
-            const int s = (it - 1) % STAGES;
-            const uint32_t par = ((it - 1) / STAGES) & 1;
             const unsigned long long t = now_ns();
-            while (!mbar_try(empty + s, par) && now_ns() - t < WAIT_LIMIT_NS) {
+            while (!mbar_try(empty + last, last_par) && now_ns() - t < WAIT_LIMIT_NS) {
             }
         }
     } else if (warp >= 4) {
         // ---------------------------------------------------------------- epilogue
         // Warp w reads TMEM lanes 32 (w % 4) .. +31 (its hardware lane quarter: one query per
-        // thread) and every EPI_PER_QUARTER-th 32-column chunk of each accumulator.
+        // thread) and the chunks part and part + EPI_PER_QUARTER of each accumulator.
         const int quarter = warp & 3;
         const int part = (warp - 4) >> 2;  // 0 .. EPI_PER_QUARTER - 1
         const int row = quarter * 32 + lane;  // TMEM lane = query row of the tile
         const int q = qt * BM + row;
-        const bool qvalid = q < p.nq;
-        const float qq = (qvalid && !I8) ? p.qq[q] : 0.f;
-        const int32_t qqi = (qvalid && I8) ? p.qqi[q] : 0;
-        const float thr = qvalid ? p.thr[q] : -INFINITY;
         const int nseg = int(gridDim.y) * EPI_PER_QUARTER;
+        EpiThread<I8> E;
+        const bool qvalid = q < p.nq, l2 = p.metric == HNSW_B200_L2;
+        const float thr = !qvalid ? -INFINITY : p.thr ? p.thr[q] : INFINITY;
+        if constexpr (I8) {
+            E.add = qvalid && l2 ? p.qqi[q] : 0;
+            E.mul = p.mul;
+            // Largest v whose float distance fl(v + add) may be <= thr: exact below 2^24; above it a
+            // float is the rounding of integers up to 64 away, so the bound is widened (a few rows
+            // beyond the threshold then join the candidates). No value for -inf or NaN.
+            const double t = double(thr);
+            const double w = floor(fmin(fmax(t, -2147483648.0), 2147483647.0)) - double(E.add) +
+                             (fabs(t) >= 16777216.0 ? 128.0 : 0.0);
+            E.thr = !(t > -INFINITY) ? INT32_MIN
+                                     : int32_t(fmax(fmin(w, double(I8_PAD - 1)), -2147483647.0));
+        } else {
+            E.add = !qvalid ? 0.f : l2 ? p.qq[q] : (p.metric == HNSW_B200_COSINE ? 1.f : 0.f);
+            E.mul = float(p.mul);
+            E.thr = thr;
+        }
         const int64_t seg = int64_t(qvalid ? q : 0) * nseg + int64_t(blockIdx.y) * EPI_PER_QUARTER + part;
-        float *cv = p.cand_val + seg * p.cap;
-        int32_t *ci = p.cand_id + seg * p.cap;
-        int cnt = 0;  // this thread's appends (its own segment: no atomics)
-        const bool l2 = p.metric == HNSW_B200_L2;
-        const bool cosine = p.metric == HNSW_B200_COSINE;
+        E.cv = p.cand_val + seg * p.cap;
+        E.ci = p.cand_id + seg * p.cap;
+        E.cap = p.cap;
+        E.cnt = 0;  // this thread's appends (its own segment: no atomics)
+        const int c0 = part * CW, c1 = c0 + CW * EPI_PER_QUARTER;
+        typename EpiThread<I8>::V bm = 0;  // threshold pass: the current block's minimum
         for (int lt = 0; lt < ntiles; lt++) {
             const int b = lt & 1;
-            const int row0 = p.row_begin + (t0 + lt) * BN;
-            int ok = 1;
-            if (lane == 0)
-                ok = (mbar_wait(tfull + b, (lt >> 1) & 1, abort_flag) &&
-                      mbar_wait(xfull + lt % XSLOTS, (lt / XSLOTS) & 1, abort_flag))
-                         ? 1
-                         : 0;
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (!ok) {
+            const int row0 = (t0 + lt) * p.tile_stride * BN;
+            const bool ok = mbar_wait(xfull + lt % XSLOTS, (lt / XSLOTS) & 1, abort_flag) &&
+                            mbar_wait(tfull + b, (lt >> 1) & 1, abort_flag);
+            if (!__all_sync(0xffffffffu, ok)) {
                 if (lane == 0) {
                     atomicExch(p.err, 1);
                     *abort_flag = 1;
@@ -451,127 +552,39 @@ __global__ void __launch_bounds__(FILTER_THREADS, 1)
             // TMEM columns of this warp's lane quarter in accumulator b; the tile's |x|^2 in its slot
             const uint32_t tbase = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(b * BN);
             const unsigned char *xslot = xring + (lt % XSLOTS) * BN * 4;
-            float tmin = INFINITY;  // threshold pass: minimum over this thread's chunks of the tile
-            bool tany = false;
-#pragma unroll 1
-            for (int c = part * CW; c < BN; c += CW * EPI_PER_QUARTER) {
-                const int col0 = row0 + c;
-                const int valid = min(CW, p.row_end - col0);  // columns that are data rows
-                // The filter value is a = v + vadd with v = |x|^2 - 2 q.x (l2), -q.x (ip, cosine)
-                // and vadd = |q|^2, 0, 1: one FMA (integer multiply-add) or negation per element,
-                // then the chunk's minimum. a is monotonic in v (float rounding included), so a
-                // chunk whose minimum fails the threshold has no candidate; the rare chunks with
-                // one test each element. |x|^2 of the CW columns comes from the tile's ring slot,
-                // which the producer filled with one bulk copy (zero beyond the data rows): the
-                // same addresses in every lane (shared-memory broadcasts) instead of an L2 round
-                // trip per chunk (the whole 1M x 128 call: 6.95 against 7.06 ms).
-                float v[CW];     // BF16 path: v; byte path: the raw S32 accumulator bits
-                int32_t w[CW];   // byte path: v, exact
-                float amin, vadd = 0.f;
-                int32_t vaddi = 0;
-                if constexpr (I8) {
-                    int32_t xv[CW];
-                    if (l2) {
-                        const int4 *x4 = reinterpret_cast<const int4 *>(xslot) + c / 4;
-#pragma unroll
-                        for (int i = 0; i < CW / 4; i++) {
-                            const int4 t = x4[i];
-                            xv[4 * i] = t.x;
-                            xv[4 * i + 1] = t.y;
-                            xv[4 * i + 2] = t.z;
-                            xv[4 * i + 3] = t.w;
-                        }
-                    }
-                    tmem_ld<CW>(tbase + uint32_t(c), v);
-#pragma unroll
-                    for (int j = 0; j < CW; j++)
-                        w[j] = l2 ? xv[j] - 2 * __float_as_int(v[j]) : -__float_as_int(v[j]);
-                    if (valid < CW) {  // uniform: only the last tile of the rows
-#pragma unroll
-                        for (int j = 0; j < CW; j++)
-                            if (j >= valid) w[j] = I8_PAD;
-                    }
-                    int32_t mh[CW / 2];
-#pragma unroll
-                    for (int j = 0; j < CW / 2; j++) mh[j] = min(w[j], w[j + CW / 2]);
-#pragma unroll
-                    for (int s2 = CW / 4; s2 > 0; s2 >>= 1)
-#pragma unroll
-                        for (int j = 0; j < s2; j++) mh[j] = min(mh[j], mh[j + s2]);
-                    vaddi = l2 ? qqi : 0;
-                    amin = float(mh[0] + vaddi);
-                } else {
-                    float xv[CW];
-                    if (l2) {
-                        const float4 *x4 = reinterpret_cast<const float4 *>(xslot) + c / 4;
-#pragma unroll
-                        for (int i = 0; i < CW / 4; i++) {
-                            const float4 t = x4[i];
-                            xv[4 * i] = t.x;
-                            xv[4 * i + 1] = t.y;
-                            xv[4 * i + 2] = t.z;
-                            xv[4 * i + 3] = t.w;
-                        }
-                    }
-                    tmem_ld<CW>(tbase + uint32_t(c), v);
-                    if (l2) {
-#pragma unroll
-                        for (int j = 0; j < CW; j++) v[j] = fmaf(-2.f, v[j], xv[j]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < CW; j++) v[j] = -v[j];
-                    }
-                    if (valid < CW) {  // uniform: only the last tile of the rows
-#pragma unroll
-                        for (int j = 0; j < CW; j++)
-                            if (j >= valid) v[j] = INFINITY;
-                    }
-                    float mh[CW / 2];
-#pragma unroll
-                    for (int j = 0; j < CW / 2; j++) mh[j] = fminf(v[j], v[j + CW / 2]);
-#pragma unroll
-                    for (int s2 = CW / 4; s2 > 0; s2 >>= 1)
-#pragma unroll
-                        for (int j = 0; j < s2; j++) mh[j] = fminf(mh[j], mh[j + s2]);
-                    vadd = l2 ? qq : (cosine ? 1.f : 0.f);
-                    amin = mh[0] + vadd;
-                }
-                if (p.block_min) {
-                    if (valid > 0) {
-                        tmin = fminf(tmin, amin);
-                        tany = true;
-                    }
-                } else if (qvalid && amin <= thr) {
-#pragma unroll
-                    for (int j = 0; j < CW; j++) {  // static indices keep v[] in registers
-                        const float a = I8 ? float(w[j] + vaddi) : v[j] + vadd;
-                        if (j < valid && a <= thr) {
-                            if (cnt < p.cap) {
-                                cv[cnt] = a;
-                                ci[cnt] = col0 + j;
-                            }
-                            cnt++;
-                        }
-                    }
-                }
-            }
-            // Threshold pass: one value per (tile, part) block, the block's minimum. The k-th
-            // smallest of the blocks' minima is at least the k-th smallest of all the values (a
-            // subset's k-th is never below the set's), so it still bounds the k-th distance from
-            // above; with far more blocks than k it is nearly as tight. Values only: the pass needs
-            // no row ids.
-            if (p.block_min && tany && qvalid) {
-                if (cnt < p.cap) cv[cnt] = tmin;
-                cnt++;
-            }
+            const int valid0 = p.row_end - row0 - c0, valid1 = p.row_end - row0 - c1;
+            uint32_t r0[CW], r1[CW];
+            typename EpiThread<I8>::V mg[CW / 4];
+            tmem_ld(tbase + uint32_t(c0), r0);
+            tmem_wait(r0);
+            tmem_ld(tbase + uint32_t(c1), r1);  // in flight while the first chunk is worked on
+            const auto m0 = E.minima(r0, xslot + c0 * 4, mg);
+            if (!BMIN && __any_sync(0xffffffffu, E.pass(m0)))
+                E.append(tbase + uint32_t(c0), xslot + c0 * 4, row0 + c0, valid0, mg);
+            tmem_wait(r1);
+            const auto m1 = E.minima(r1, xslot + c1 * 4, mg);
+            if (!BMIN && __any_sync(0xffffffffu, E.pass(m1)))
+                E.append(tbase + uint32_t(c1), xslot + c1 * 4, row0 + c1, valid1, mg);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(tempty + b);
                 mbar_arrive(xempty + lt % XSLOTS);
             }
+            // Threshold pass: one value per block, the minimum of this thread's chunks of two tiles. The
+            // r-th smallest of the blocks' minima is at least the r-th smallest of all the values (a
+            // subset's r-th is never below the set's); with far more blocks than r it is nearly as tight.
+            // Values only: the pass needs no row ids.
+            if constexpr (BMIN) {
+                const auto m = min2(m0, m1);
+                bm = b == 0 ? m : min2(bm, m);
+                if ((b == 1 || lt + 1 == ntiles) && qvalid) {
+                    if (E.cnt < E.cap) E.cv[E.cnt] = float(bm + E.add);
+                    E.cnt++;
+                }
+            }
         }
-        if (qvalid) p.cand_cnt[seg] = cnt;
+        if (qvalid) p.cand_cnt[seg] = E.cnt;
     }
     __syncthreads();
     if (warp == 2) {
@@ -582,80 +595,113 @@ __global__ void __launch_bounds__(FILTER_THREADS, 1)
 }
 
 // ------------------------------------------------------------------------------------- prep
-// Byte rows (values checked to be integers in [0, 255]): one warp per row writes the u8 operand row
-// of width kpad (a multiple of 128, zero past dim), four bytes a lane, and the exact |x|^2.
+// Four values of a byte row from element i, as bytes of a word (zero past dim). vec: the row starts on a
+// boundary of four elements and dim is a multiple of 4, so one load fetches them.
+__device__ __forceinline__ uint32_t byte_word(const uint8_t *x, int i, int dim, bool vec) {
+    if (vec) return i < dim ? __ldg(reinterpret_cast<const uint32_t *>(x + i)) : 0u;
+    uint32_t word = 0;
+#pragma unroll
+    for (int t = 0; t < 4; t++) word |= (i + t < dim ? uint32_t(x[i + t]) : 0u) << (8 * t);
+    return word;
+}
+__device__ __forceinline__ uint32_t byte_word(const float *x, int i, int dim, bool vec) {
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (vec && i < dim) {
+        const float4 f = __ldg(reinterpret_cast<const float4 *>(x + i));
+        v[0] = f.x;
+        v[1] = f.y;
+        v[2] = f.z;
+        v[3] = f.w;
+    } else if (!vec) {
+#pragma unroll
+        for (int t = 0; t < 4; t++)
+            if (i + t < dim) v[t] = x[i + t];
+    }
+    uint32_t word = 0;
+#pragma unroll
+    for (int t = 0; t < 4; t++) word |= uint32_t(int32_t(v[t]) & 255) << (8 * t);
+    return word;
+}
+
+// Byte rows (values checked to be integers in [0, 255]): a warp writes the u8 operand rows of width
+// kpad (a multiple of 128, zero past dim), four bytes a lane, and sq: the exact |x|^2 (norms; else 0; `past` beyond the rows), four rows at a time
+// so that their loads overlap (bound by memory: 1M x 128 bytes 112 -> 71 us, a row and a byte at a time before).
 template <typename T>
 __global__ void prep_rows_u8(const T *src, int64_t rows, int dim, int64_t rows_pad, int kpad,
-                             uint8_t *dst, int32_t *sq) {
+                             uint8_t *dst, int32_t *sq, bool vec, bool norms, int32_t past) {
+    constexpr int R = 4;
     const int lane = threadIdx.x & 31;
-    const int64_t wpb = blockDim.x >> 5;
-    for (int64_t r = int64_t(blockIdx.x) * wpb + (threadIdx.x >> 5); r < rows_pad;
-         r += int64_t(gridDim.x) * wpb) {
-        uint32_t *out = reinterpret_cast<uint32_t *>(dst + r * kpad);
-        const T *x = src + r * dim;
-        int32_t ss = 0;
+    const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
+    for (int64_t r = (int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * R; r < rows_pad;
+         r += warps * R) {
+        uint32_t ss[R] = {0u, 0u, 0u, 0u};
         for (int i = lane * 4; i < kpad; i += 128) {
-            uint32_t word = 0;
+            uint32_t w[R];
 #pragma unroll
-            for (int t = 0; t < 4; t++) {
-                const int32_t v = (r < rows && i + t < dim) ? int32_t(x[i + t]) : 0;
-                ss += v * v;
-                word |= uint32_t(v & 255) << (8 * t);
+            for (int t = 0; t < R; t++) w[t] = r + t < rows ? byte_word(src + (r + t) * dim, i, dim, vec) : 0u;
+#pragma unroll
+            for (int t = 0; t < R; t++) {
+                ss[t] = __dp4a(w[t], w[t], ss[t]);
+                if (r + t < rows_pad) *reinterpret_cast<uint32_t *>(dst + (r + t) * kpad + i) = w[t];
             }
-            out[i >> 2] = word;
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (lane == 0) sq[r] = ss;
+        for (int t = 0; t < R; t++) {
+            const uint32_t sum = __reduce_add_sync(0xffffffffu, ss[t]);
+            if (lane == 0 && r + t < rows_pad) sq[r + t] = r + t >= rows ? past : norms ? int32_t(sum) : 0;
+        }
     }
 }
 
-// One warp per row: float64 norm, cosine normalisation, BF16 operand row(s) of width kpad.
-// terms == 1: [v]; terms == 3: A-side [hi, hi, lo] (queries) or B-side [hi, lo, hi] (data).
+// One warp per row: float64 norm, cosine normalisation, BF16 operand row(s) of width kpad, and sq32:
+// |x|^2 (norms; else 0; `past` beyond the rows). terms == 1: [v]; terms == 3: A-side [hi, hi, lo]
+// (queries) or B-side [hi, lo, hi] (data). A lane keeps up to PREP_REGS values of its row in registers, so
+// that a value is read once (bound by memory and the row's latency; 200K x 100 floats: 86 -> 65 us, and
+// 105 us with four rows a warp).
+constexpr int PREP_REGS = 4;
 template <typename T>
 __global__ void prep_rows(const T *src, int64_t rows, int dim, int64_t rows_pad, int kpad,
                           int terms, int a_side, int cosine, __nv_bfloat16 *dst, double *norm64,
-                          float *sq32) {
+                          float *sq32, bool norms, float past) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
     const int seg = kpad / terms;  // padded dim per term
     for (int64_t r = warp; r < rows_pad; r += nwarps) {
-        __nv_bfloat16 *out = dst + r * kpad;
-        if (r >= rows) {
-            for (int i = lane; i < kpad; i += 32) out[i] = __float2bfloat16(0.f);
-            if (lane == 0) {
-                norm64[r] = 0.0;
-                sq32[r] = 0.f;
-            }
-            continue;
-        }
-        const T *x = src + r * dim;
+        const T *xr = src + r * dim;
+        auto value = [&](int i) { return r < rows && i < dim ? float(xr[i]) : 0.f; };
+        float x[PREP_REGS];
+#pragma unroll
+        for (int t = 0; t < PREP_REGS; t++) x[t] = value(lane + 32 * t);
         double ss = 0.0;
-        for (int i = lane; i < dim; i += 32) {
-            const double v = double(x[i]);
+#pragma unroll
+        for (int t = 0; t < PREP_REGS; t++) ss += double(x[t]) * double(x[t]);
+        for (int i = lane + 32 * PREP_REGS; i < dim; i += 32) {
+            const double v = double(value(i));
             ss += v * v;
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
         const double nrm = sqrt(ss);
         const double scale = cosine ? (nrm > 0 ? 1.0 / nrm : 0.0) : 1.0;
-        for (int i = lane; i < seg; i += 32) {
-            const double v = i < dim ? double(x[i]) * scale : 0.0;
-            const float vf = float(v);
-            const __nv_bfloat16 hi = __float2bfloat16_rn(vf);
-            if (terms == 1) {
-                out[i] = hi;
-            } else {
+        __nv_bfloat16 *out = dst + r * kpad;
+        auto put = [&](int i, float raw) {
+            const double v = double(raw) * scale;
+            const __nv_bfloat16 hi = __float2bfloat16_rn(float(v));
+            out[i] = hi;
+            if (terms != 1) {
                 const __nv_bfloat16 lo = __float2bfloat16_rn(float(v - double(__bfloat162float(hi))));
-                out[i] = hi;
                 out[seg + i] = a_side ? hi : lo;
                 out[2 * seg + i] = a_side ? lo : hi;
             }
-        }
+        };
+#pragma unroll
+        for (int t = 0; t < PREP_REGS; t++)
+            if (lane + 32 * t < seg) put(lane + 32 * t, x[t]);
+        for (int i = lane + 32 * PREP_REGS; i < seg; i += 32) put(i, value(i));
         if (lane == 0) {
             norm64[r] = nrm;  // cosine rerank re-normalises with it; margins use 1 for cosine
-            sq32[r] = cosine ? 1.f : float(ss);
+            sq32[r] = r >= rows ? past : norms ? float(ss) : 0.f;
         }
     }
 }
@@ -724,9 +770,14 @@ __device__ __forceinline__ int compact_list(float *v, int32_t *id, const int32_t
 constexpr int SELECT_WARPS = 8;
 // The query's list is first compacted in place (compact_list) and its length stored in
 // cand_m[q], so the radix passes and the re-rank read one dense run of entries.
+// final_pass: the list is pass two's, out_tau holds the threshold it was collected with (without the
+// margin), and *short_lists is set when that threshold turns out too low: fewer than k entries, or
+// a k-th smallest above it. stat_max: largest |value| the error bound is stated for (byte rows: the
+// finite final thresholds; else the margins), as float bits.
 __global__ void select_kth(float *cand_val, int32_t *cand_id, const int32_t *cand_cnt, int32_t cap,
                            int32_t nseg, int32_t nq, int32_t k, const float *margin, float *out_thr,
-                           float *out_tau, int32_t *cand_m) {
+                           float *out_tau, int32_t *cand_m, int final_pass, int bytes,
+                           int32_t *short_lists, unsigned int *stat_max) {
     __shared__ uint32_t hist_all[SELECT_WARPS][256];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q = blockIdx.x * SELECT_WARPS + wid;
@@ -738,6 +789,7 @@ __global__ void select_kth(float *cand_val, int32_t *cand_id, const int32_t *can
     if (lane == 0) cand_m[q] = m;
     if (m < k) {
         if (lane == 0) {
+            if (final_pass) atomicOr(short_lists, 1);
             out_tau[q] = INFINITY;
             out_thr[q] = INFINITY;
         }
@@ -785,9 +837,15 @@ __global__ void select_kth(float *cand_val, int32_t *cand_id, const int32_t *can
         __syncwarp();
     }
     if (lane == 0) {
-        const float tau = funkey(prefix);
+        const float tau = funkey(prefix), mg = margin[q];
+        if (final_pass) {
+            if (!(tau <= out_tau[q])) atomicOr(short_lists, 1);
+            const float b = bytes ? fabsf(tau + mg) : mg;
+            const unsigned int bits = isfinite(b) || !bytes ? __float_as_uint(b) : 0u;
+            if (bits > *static_cast<volatile unsigned int *>(stat_max)) atomicMax(stat_max, bits);
+        }
         out_tau[q] = tau;
-        out_thr[q] = tau + margin[q];
+        out_thr[q] = tau + mg;
     }
 }
 
@@ -817,6 +875,43 @@ __device__ __forceinline__ double dist_f64_lane(const T *x, const T *qv, int dim
     return __dsub_rn(1.0, acc);
 }
 
+// Float64 distances of up to 32 rows (ids[0 .. m) in shared memory) with the same sums in dimension
+// order: the warp computes the products of 32 dimensions of every row together (coalesced loads; under
+// cosine the two divisions of each product, which are most of the work, spread over the lanes), then
+// lane s adds row s's products in order. qs: the query's values (cosine: divided by its norm) in
+// shared memory; P: 32 rows of DIST_PITCH doubles. Lane s < m returns its row's distance.
+constexpr int DIST_PITCH = 33;
+template <typename T>
+__device__ __forceinline__ double dist_f64_rows(const T *data, const int32_t *ids, int m, const double *qs,
+                                                int dim, int metric, const double *xnorm, double *P,
+                                                int lane) {
+    double acc = 0.0;
+    for (int d0 = 0; d0 < dim; d0 += 32) {
+        const int d = d0 + lane;
+        const double qd = d < dim ? qs[d] : 0.0;
+        for (int s = 0; s < m; s++) {
+            const int64_t id = ids[s];
+            double pr = 0.0;
+            if (d < dim) {
+                const double x = double(data[id * dim + d]);
+                if (metric == HNSW_B200_L2) {
+                    const double df = __dsub_rn(x, qd);
+                    pr = __dmul_rn(df, df);
+                } else {
+                    pr = __dmul_rn(metric == HNSW_B200_IP ? x : __ddiv_rn(x, xnorm[id]), qd);
+                }
+            }
+            P[s * DIST_PITCH + lane] = pr;
+        }
+        __syncwarp();
+        const int nd = min(32, dim - d0);
+        if (lane < m)
+            for (int j = 0; j < nd; j++) acc = __dadd_rn(acc, P[lane * DIST_PITCH + j]);
+        __syncwarp();
+    }
+    return metric == HNSW_B200_L2 ? acc : (metric == HNSW_B200_IP ? -acc : __dsub_rn(1.0, acc));
+}
+
 // The same by the whole warp (long rows): lane l sums dimensions l, l + 32, ..., then a fixed
 // shuffle tree adds the lanes (the same value on every run; on integer data every order gives the
 // same exact sum), so the float64 chains are 32 times shorter. The result is on every lane.
@@ -840,8 +935,26 @@ __device__ __forceinline__ double dist_f64_warp(const T *x, const T *qv, int dim
     return metric == HNSW_B200_L2 ? acc : (metric == HNSW_B200_IP ? -acc : __dsub_rn(1.0, acc));
 }
 
+// Survivors (candidates within the final threshold) of a query that rerank_topk gathers in shared
+// memory and sorts there; a query with more (many exact ties) inserts them one by one.
+__host__ __device__ constexpr int survivor_slots(int k) { return k + k / 4 + 64; }
+// Shared memory of one warp of rerank_topk: distances and ids of the results and of the survivors,
+// then (rows below COOP_DIM re-scored in float64) the query and a block of products.
+__host__ __device__ inline size_t rerank_smem(int k, int dim, bool gather, bool products) {
+    size_t b = size_t(k + 1 + (gather ? survivor_slots(k) : 0)) * 12;
+    b = (b + 15) & ~size_t(15);
+    if (products) b += size_t(dim) * 8 + size_t(32) * DIST_PITCH * 8;
+    return (b + 15) & ~size_t(15);
+}
+
 // One warp per query: exact float64 distances of the candidates within the final threshold,
-// best k by (distance, id) kept in shared memory (sorted insertion), written as int64 / float64.
+// best k by (distance, id), written as int64 / float64.
+// gather: the survivors are first collected in shared memory (most candidates fail the final threshold:
+// scored in batches of candidates, a float64 chain ran for one or two of 32 lanes), scored 32 at a
+// time and placed by counting the ones below each: about k^2 / 32 steps, against k insertions of about 80
+// instructions. 10K queries x 1M x 128 bytes, k = 100: 332 -> 102 us; 1,000 x 200K x 100 cosine,
+// k = 10: 156 -> 33 us. Without room (k of several thousand) or with more survivors than slots
+// (ties), sorted insertion.
 // exact_lim > 0 (byte rows, integer filter): a candidate whose filter value is below exact_lim in
 // magnitude already holds its exact distance and is not re-scored; one result in VERIFY_EVERY of
 // every query (positions q, q + VERIFY_EVERY, ... mod VERIFY_EVERY, so a batch covers every
@@ -854,15 +967,19 @@ __global__ void rerank_topk(const T *data, const T *queries, int dim, int32_t nq
                             const float *cand_val, const int32_t *cand_id, const int32_t *cand_m,
                             int32_t cap, int32_t nseg, const float *thr, int64_t *out_ids,
                             double *out_d, unsigned long long *err_max, float exact_lim,
-                            int32_t *mismatch) {
+                            int32_t *mismatch, int gather, int products) {
     extern __shared__ __align__(16) unsigned char sm[];
-    const int warps = blockDim.x >> 5;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int q = blockIdx.x * warps + w;
-    double *Ad = reinterpret_cast<double *>(sm) + size_t(w) * (k + 1);
-    int32_t *Ai = reinterpret_cast<int32_t *>(reinterpret_cast<double *>(sm) + size_t(warps) * (k + 1)) +
-                  size_t(w) * (k + 1);
-    if (q >= nq) return;
+    const int q = blockIdx.x * (blockDim.x >> 5) + w;
+    if (q >= nq) return;  // no block-wide barrier below
+    const int slots = gather ? survivor_slots(k) : 0;
+    unsigned char *base = sm + size_t(w) * rerank_smem(k, dim, gather, products);
+    double *Ad = reinterpret_cast<double *>(base);       // results
+    double *Sd = Ad + k + 1;                             // survivors
+    int32_t *Ai = reinterpret_cast<int32_t *>(Sd + slots);
+    int32_t *Si = Ai + k + 1;
+    double *qs = reinterpret_cast<double *>(base + rerank_smem(k, dim, gather, false));
+    double *P = qs + dim;
     const float t = thr[q];
     const T *qv = queries + int64_t(q) * dim;
     const bool cos = metric == HNSW_B200_COSINE;
@@ -873,57 +990,123 @@ __global__ void rerank_topk(const T *data, const T *queries, int dim, int32_t nq
     // one per lane.
     const int m = cand_m[q];
     const int64_t region = int64_t(q) * nseg * cap;
-    for (int b0 = 0; b0 < m; b0 += 32) {
-        const int64_t at = b0 + lane < m ? region + b0 + lane : -1;  // this lane's entry
-        const float approx = at >= 0 ? cand_val[at] : INFINITY;
-        const bool has = at >= 0 && approx <= t;
-        const int32_t id = has ? cand_id[at] : -1;
-        const bool known = has && fabsf(approx) < exact_lim;  // exact already (byte rows)
-        const bool need = has && !known;
-        double d = known ? double(approx) : INFINITY;
-        if (dim >= COOP_DIM) {
-            for (uint32_t hm = __ballot_sync(0xffffffffu, need); hm; hm &= hm - 1) {
-                const int j = __ffs(hm) - 1;
-                const int32_t idj = __shfl_sync(0xffffffffu, id, j);
-                const double dd = dist_f64_warp(data + int64_t(idj) * dim, qv, dim, metric,
-                                                cos ? xnorm[idj] : 1.0, qn, lane);
-                if (lane == j) d = dd;
+    int ns = -1;  // survivors gathered (-1: insert one by one)
+    if (gather) {
+        ns = 0;
+        for (int b0 = 0; b0 < m; b0 += 32) {
+            const bool in = b0 + lane < m;
+            const float approx = in ? cand_val[region + b0 + lane] : INFINITY;
+            const bool has = in && approx <= t;
+            const uint32_t hm = __ballot_sync(0xffffffffu, has);
+            const int at = ns + __popc(hm & ((1u << lane) - 1u));
+            if (has && at < slots) {
+                Sd[at] = double(approx);
+                Si[at] = cand_id[region + b0 + lane];
             }
-        } else if (need) {
-            d = dist_f64_lane(data + int64_t(id) * dim, qv, dim, metric, cos ? xnorm[id] : 1.0, qn);
+            ns += __popc(hm);
+            if (ns > slots) break;  // uniform
         }
-        if (need) err = fmax(err, fabs(double(approx) - d));
-        uint32_t am = __ballot_sync(0xffffffffu, has);
-        while (am) {
-            const int j = __ffs(am) - 1;
-            am &= am - 1;
-            const double xd = __shfl_sync(0xffffffffu, d, j);
-            const int32_t xi = __shfl_sync(0xffffffffu, id, j);
-            if (a == k && !pair_lt(xd, xi, Ad[k - 1], Ai[k - 1])) continue;
-            int c = 0;
-            for (int r = lane; r < a; r += 32) c += pair_lt(Ad[r], Ai[r], xd, xi);
-            const int pos = __reduce_add_sync(0xffffffffu, c);
-            for (int top = a - 1; top >= pos; top -= 32) {
-                const int r = top - lane;
-                double dv = 0;
-                int32_t iv = 0;
-                if (r >= pos) {
-                    dv = Ad[r];
-                    iv = Ai[r];
+        if (ns > slots) ns = -1;
+        __syncwarp();
+    }
+    if (ns >= 0) {
+        if (products && !cos)
+            for (int i = lane; i < dim; i += 32) qs[i] = double(qv[i]);
+        if (products && cos)
+            for (int i = lane; i < dim; i += 32) qs[i] = __ddiv_rn(double(qv[i]), qn);
+        __syncwarp();
+        for (int b0 = 0; b0 < ns; b0 += 32) {
+            const int s = b0 + lane;
+            const double approx = s < ns ? Sd[s] : 0.0;
+            const bool need = s < ns && !(fabs(approx) < double(exact_lim));
+            const uint32_t nm = __ballot_sync(0xffffffffu, need);
+            if (!nm) continue;  // uniform
+            double d = approx;
+            if (dim >= COOP_DIM) {
+                for (uint32_t hm = nm; hm; hm &= hm - 1) {
+                    const int j = __ffs(hm) - 1;
+                    const int32_t idj = Si[b0 + j];
+                    const double dd = dist_f64_warp(data + int64_t(idj) * dim, qv, dim, metric,
+                                                    cos ? xnorm[idj] : 1.0, qn, lane);
+                    if (lane == j) d = dd;
+                }
+            } else if (products) {
+                const double dd = dist_f64_rows(data, Si + b0, min(32, ns - b0), qs, dim, metric, xnorm, P, lane);
+                if (need) d = dd;
+            } else if (need) {  // byte rows: distances of 2^24 or more only
+                d = dist_f64_lane(data + int64_t(Si[s]) * dim, qv, dim, metric, cos ? xnorm[Si[s]] : 1.0, qn);
+            }
+            if (need) {
+                err = fmax(err, fabs(approx - d));
+                Sd[s] = d;
+            }
+        }
+        __syncwarp();
+        for (int s = lane; s < ns; s += 32) {
+            const double d = Sd[s];
+            const int32_t id = Si[s];
+            int pos = 0;
+            for (int j = 0; j < ns; j++) pos += pair_lt(Sd[j], Si[j], d, id);
+            if (pos < k) {
+                Ad[pos] = d;
+                Ai[pos] = id;
+            }
+        }
+        a = min(ns, k);
+        __syncwarp();
+    } else {
+        for (int b0 = 0; b0 < m; b0 += 32) {
+            const int64_t at = b0 + lane < m ? region + b0 + lane : -1;  // this lane's entry
+            const float approx = at >= 0 ? cand_val[at] : INFINITY;
+            const bool has = at >= 0 && approx <= t;
+            const int32_t id = has ? cand_id[at] : -1;
+            const bool known = has && fabsf(approx) < exact_lim;  // exact already (byte rows)
+            const bool need = has && !known;
+            double d = known ? double(approx) : INFINITY;
+            if (dim >= COOP_DIM) {
+                for (uint32_t hm = __ballot_sync(0xffffffffu, need); hm; hm &= hm - 1) {
+                    const int j = __ffs(hm) - 1;
+                    const int32_t idj = __shfl_sync(0xffffffffu, id, j);
+                    const double dd = dist_f64_warp(data + int64_t(idj) * dim, qv, dim, metric,
+                                                    cos ? xnorm[idj] : 1.0, qn, lane);
+                    if (lane == j) d = dd;
+                }
+            } else if (need) {
+                d = dist_f64_lane(data + int64_t(id) * dim, qv, dim, metric, cos ? xnorm[id] : 1.0, qn);
+            }
+            if (need) err = fmax(err, fabs(double(approx) - d));
+            uint32_t am = __ballot_sync(0xffffffffu, has);
+            while (am) {
+                const int j = __ffs(am) - 1;
+                am &= am - 1;
+                const double xd = __shfl_sync(0xffffffffu, d, j);
+                const int32_t xi = __shfl_sync(0xffffffffu, id, j);
+                if (a == k && !pair_lt(xd, xi, Ad[k - 1], Ai[k - 1])) continue;
+                int c = 0;
+                for (int r = lane; r < a; r += 32) c += pair_lt(Ad[r], Ai[r], xd, xi);
+                const int pos = __reduce_add_sync(0xffffffffu, c);
+                for (int top = a - 1; top >= pos; top -= 32) {
+                    const int r = top - lane;
+                    double dv = 0;
+                    int32_t iv = 0;
+                    if (r >= pos) {
+                        dv = Ad[r];
+                        iv = Ai[r];
+                    }
+                    __syncwarp();
+                    if (r >= pos) {
+                        Ad[r + 1] = dv;
+                        Ai[r + 1] = iv;
+                    }
+                    __syncwarp();
+                }
+                if (lane == 0) {
+                    Ad[pos] = xd;
+                    Ai[pos] = xi;
                 }
                 __syncwarp();
-                if (r >= pos) {
-                    Ad[r + 1] = dv;
-                    Ai[r + 1] = iv;
-                }
-                __syncwarp();
+                a = min(a + 1, k);
             }
-            if (lane == 0) {
-                Ad[pos] = xd;
-                Ai[pos] = xi;
-            }
-            __syncwarp();
-            a = min(a + 1, k);
         }
     }
     if (exact_lim > 0.f) {  // results r = q, q + VERIFY_EVERY, ... (mod VERIFY_EVERY) in float64
@@ -957,15 +1140,25 @@ __global__ void rerank_topk(const T *data, const T *queries, int dim, int32_t nq
 // branches and an integer OR across the warp: a form that combined two boolean warp votes set the
 // wrong bits on the GPU (every non-integer and 300 read as bytes), this one was checked against
 // those values there.
+__device__ __forceinline__ int value_class(float v) {
+    int f = 0;
+    const float r = rintf(v);
+    if (r != v || !(fabsf(v) <= 256.f)) f |= 1;
+    if (r != v || !(v >= 0.f) || !(v <= 255.f)) f |= 2;
+    return f;
+}
+
 __global__ void check_small_int(const float *x, int64_t count, int32_t *flag) {
     int f = 0;
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count;
-         i += int64_t(gridDim.x) * blockDim.x) {
-        const float v = x[i];
-        const float r = rintf(v);
-        if (r != v || !(fabsf(v) <= 256.f)) f |= 1;
-        if (r != v || !(v >= 0.f) || !(v <= 255.f)) f |= 2;
+    const int64_t at = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, step = int64_t(gridDim.x) * blockDim.x;
+    const int64_t n4 = (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? count >> 2 : 0;  // 16-byte pieces
+    const float4 *x4 = reinterpret_cast<const float4 *>(x);
+#pragma unroll 4
+    for (int64_t i = at; i < n4; i += step) {
+        const float4 v = __ldg(x4 + i);
+        f |= value_class(v.x) | value_class(v.y) | value_class(v.z) | value_class(v.w);
     }
+    for (int64_t i = 4 * n4 + at; i < count; i += step) f |= value_class(x[i]);
     f = int(__reduce_or_sync(0xffffffffu, uint32_t(f)));
     if (f && (threadIdx.x & 31) == 0) atomicOr(flag, f);
 }
@@ -1080,27 +1273,46 @@ size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Candidate lists take at most CAND_BYTES of scratch: (query, segment) pairs x cap x 8 bytes.
 constexpr int64_t CAND_BYTES = int64_t(4) << 30;
-// Pass two keeps about k n / prefix rows per query: tau is the k-th smallest of the prefix's CW-row
-// block minima, a loose upper bound of the k-th distance (830 per query measured for k = 100 on the
-// 1M x 128 mixture with a prefix of n / 8, against 800 for k n / prefix). Lists are sized for
-// EXPECT_FACTOR times that.
-#ifndef HB_EXPECT_FACTOR
-#define HB_EXPECT_FACTOR 2
-#endif
-constexpr int64_t EXPECT_FACTOR = HB_EXPECT_FACTOR;
+constexpr int64_t MAX_CHUNK = 16384;  // queries of a batch filtered together
+// Lists are sized for EXPECT_FACTOR times the candidates that pass two is expected to keep.
+constexpr int64_t EXPECT_FACTOR = 2;
 // Byte rows use the integer filter (1) or the BF16 one (0).
 #ifndef HB_EXACT_I8
 #define HB_EXACT_I8 1
 #endif
 // Longest byte row of the integer filter: 2 dim 255^2 stays below 2^31.
 constexpr int MAX_DIM_I8 = 8192;
-// Prefix length. Pass one costs the prefix's rows on the tensor cores; pass two then keeps about
-// k n / prefix rows per query, each re-scored in float64 (and a per-element epilogue path on the
-// chunks holding them). A float64 re-score of a row costs about PREFIX_BALANCE times a row of
-// tensor-core filter work, so the prefix balancing the two is sqrt(PREFIX_BALANCE k n): 122K rows
-// for k = 100 over 1M rows (830 candidates per query), 30K over 60K rows.
-constexpr double PREFIX_BALANCE = 150.0;
+// Pass one filters a sample: every tile_stride-th tile of the data, about sqrt(SAMPLE_BALANCE k n)
+// rows (a longer sample costs filter time, a shorter one gives a looser threshold and pass two more
+// candidates to append, select from and re-rank). Both passes with their selects and the re-rank, 10K
+// queries x 1M x 128 bytes, k = 100: 2.91 ms at 25, 2.81 at 60, 2.82 at 150, 2.91 at 300.
+constexpr double SAMPLE_BALANCE = 75.0;
 
+// Which of a sample's smallest values is the threshold. A sample of a share f of the rows holds about
+// k f of the k nearest, with a deviation of at most sqrt(k f), so its (k f + 6 sqrt(k f) + 8)-th
+// smallest lies beyond the k-th nearest of all rows but for about one query in 10^9, while only about
+// (k f + 6 sqrt(k f) + 8) / f rows pass it (at k = 100, f = 1/8: 330; the sample's k-th
+// smallest, which is never too low, let 830 pass). Pass two counts: where a threshold was too low after
+// all (rows in an order that the stride resonates with) the chunk runs again with the k-th smallest.
+int sample_rank(int64_t k, int64_t sample_tiles, int64_t tiles) {
+    if (sample_tiles >= tiles) return int(k);
+    const double mean = double(k) * double(sample_tiles) / double(tiles);
+    return int(std::min<double>(double(k), std::ceil(mean + 6.0 * std::sqrt(mean) + 8.0)));
+}
+
+// What the kernels report to the host, read once per chunk.
+struct Stats {
+    // of the current chunk
+    int32_t err;         // a bounded wait expired
+    int32_t mismatch;    // an integer filter distance differs from its float64 re-score
+    int32_t short_lists; // a sampled threshold was too low
+    int32_t pad;
+    unsigned long long longest, total;  // candidate segments
+    // of the call
+    unsigned long long filter_err;  // largest |filter value - distance|, as bits of the double
+    unsigned int bound;             // largest value the error bound is stated for, as bits of the float
+    unsigned int pad2;
+};
 
 // One attempt at the whole batch with candidate lists of at least cap_min entries. Returns
 // HNSW_B200_ERETRY with *cap_needed set when a query's candidates outgrew its list (many rows
@@ -1142,41 +1354,51 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
 
-    // Split geometry of a pass over `rows` rows for a chunk of nqc queries: the rows are split so
-    // that the chunk's query tiles fill the GPU (about four CTAs per SM).
+    // Split geometry of a pass over `tiles` tiles for a chunk of nqc queries: a CTA takes tps tiles of
+    // one query tile, and the split is the one whose waves of CTAs (one an SM) end soonest, a CTA's
+    // start and end counted as FIXED_TILES tiles.
+    constexpr int FIXED_TILES = 3;
     struct Geo {
         int tps, splits;
     };
-    auto geo = [&](int64_t nqc, int64_t rows) {
+    auto geo = [&](int64_t nqc, int tiles) {
         const int qt = int((nqc + BM - 1) / BM);
-        const int tiles = int((rows + BN - 1) / BN);
-        const int want = std::max(1, (4 * sms + qt - 1) / qt);
-        Geo g;
-        g.tps = std::max(1, (tiles + want - 1) / want);
-        g.splits = (tiles + g.tps - 1) / g.tps;
+        const int most = std::min(tiles, std::max(1, (8 * sms + qt - 1) / qt));
+        Geo g{tiles, 1};
+        int64_t best = INT64_MAX;
+        for (int s = 1; s <= most; s++) {
+            const int tps = (tiles + s - 1) / s, splits = (tiles + tps - 1) / tps;
+            const int64_t waves = (int64_t(qt) * splits + sms - 1) / sms, cost = waves * (tps + FIXED_TILES);
+            if (cost < best) {
+                best = cost;
+                g = Geo{tps, splits};
+            }
+        }
         return g;
     };
-    // Pass one keeps the minimum of every (tile, epilogue part) block of a prefix (every row when
-    // the prefix has fewer than k such blocks in whole tiles); pass two keeps the rows within tau +
-    // margin, about EXPECT_FACTOR k n / prefix of them. Each epilogue thread appends to its own
-    // segment of the query's list: in pass one at most one entry per tile (block minima) or CW
-    // (rows) per chunk it takes of a tile; pass two's segments are sized for three times their
-    // expected share (an overflow re-runs the call with longer segments).
-    const int64_t prefix = std::min<int64_t>(
-        n, std::max<int64_t>(int64_t(64) * k, int64_t(std::sqrt(PREFIX_BALANCE * double(k) * double(n)))));
-    const bool block_min = prefix / BN * EPI_PER_QUARTER >= k;
-    const int64_t expect2 = EXPECT_FACTOR * int64_t(k) * ((n + prefix - 1) / prefix) + int64_t(k);
-    int64_t QB = std::min<int64_t>(nq_all, 8192);  // queries per chunk
-    int64_t cap = 0, slots = 0;                      // entries per segment; (query, segment) pairs
+    // Pass one keeps the minimum of every block of two tiles' chunks of an epilogue thread (every row when
+    // the sample has fewer than k blocks); pass two keeps the rows within tau + margin. Each epilogue
+    // thread appends to its own segment of the query's list: in pass one at most one entry per block
+    // or its 2 CW columns of a tile; pass two's segments are sized for three times their expected share
+    // (an overflow re-runs the call with longer segments).
+    const int tiles = int((n + BN - 1) / BN);
+    const int64_t sample_rows = std::min<int64_t>(
+        n, std::max<int64_t>(int64_t(64) * k, int64_t(std::sqrt(SAMPLE_BALANCE * double(k) * double(n)))));
+    const int stride = std::max<int>(1, int(tiles / ((sample_rows + BN - 1) / BN)));
+    const int sample = (tiles + stride - 1) / stride;  // tiles 0, stride, 2 stride, ... of pass one
+    const bool block_min = int64_t(sample) / 2 * EPI_PER_QUARTER >= k;
+    const int rank = sample_rank(k, sample, tiles);
+    const int64_t expect2 = EXPECT_FACTOR * (int64_t(rank) * tiles / sample) + int64_t(k);
+    int64_t QB = std::min<int64_t>(nq_all, MAX_CHUNK);  // queries per chunk
+    int64_t cap = 0, slots = 0;                           // entries per segment; (query, segment) pairs
     for (;;) {
         cap = std::min<int64_t>(cap_min, n);
         slots = 0;
         const int64_t last = nq_all % QB ? nq_all % QB : QB;
         for (int64_t nqc : {QB, last}) {
-            const Geo g1 = geo(nqc, prefix), g2 = geo(nqc, n);
+            const Geo g1 = geo(nqc, sample), g2 = geo(nqc, tiles);
             const int64_t nseg2 = int64_t(g2.splits) * EPI_PER_QUARTER;
-            const int64_t per_tile = (BN / CW + EPI_PER_QUARTER - 1) / EPI_PER_QUARTER;  // chunks
-            cap = std::max<int64_t>(cap, per_tile * (block_min ? 1 : CW) * g1.tps);
+            cap = std::max<int64_t>(cap, block_min ? (g1.tps + 1) / 2 : int64_t(2 * CW) * g1.tps);
             cap = std::max<int64_t>(cap, (3 * expect2 + nseg2 - 1) / nseg2 + 32);
             slots = std::max<int64_t>(slots, nqc * std::max(g1.splits, g2.splits) * EPI_PER_QUARTER);
         }
@@ -1205,10 +1427,8 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
     const size_t o_cm = carve(size_t(QB) * 4);
     const size_t o_cv = carve(size_t(slots) * cap * 4);
     const size_t o_ci = carve(size_t(slots) * cap * 4);
-    const size_t o_cs = carve(16);
-    const size_t o_err = carve(16);
+    const size_t o_st = carve(sizeof(Stats));
     const size_t o_mx = carve(16);
-    const size_t o_fe = carve(16);
     if (int rc = buf.get(off)) return rc;
     char *B = static_cast<char *>(buf.p);
     auto *xb = reinterpret_cast<__nv_bfloat16 *>(B + o_xb);
@@ -1228,17 +1448,20 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
     auto *cm = reinterpret_cast<int32_t *>(B + o_cm);  // per query: candidates after compaction
     auto *cv = reinterpret_cast<float *>(B + o_cv);
     auto *ci = reinterpret_cast<int32_t *>(B + o_ci);
-    auto *err = reinterpret_cast<int32_t *>(B + o_err);
+    auto *st = reinterpret_cast<Stats *>(B + o_st);
     const T *X = static_cast<const T *>(a->data);
     const int cos = metric == HNSW_B200_COSINE;
+    const bool l2 = metric == HNSW_B200_L2;
     int64_t launches = 0;
 
+    // rows that can be read four elements a load
+    auto vec = [&](const T *p) { return (dim & 3) == 0 && reinterpret_cast<uintptr_t>(p) % (4 * sizeof(T)) == 0; };
     if (bytes)
-        prep_rows_u8<T><<<int(std::min<int64_t>(4096, (n_pad + 7) / 8)), 256, 0, s>>>(
-            X, n, dim, n_pad, kp, xb8, xxi);
+        prep_rows_u8<T><<<int(std::min<int64_t>(4096, (n_pad + 31) / 32)), 256, 0, s>>>(
+            X, n, dim, n_pad, kp, xb8, xxi, vec(X), l2, I8_PAD);
     else
-        prep_rows<T><<<int(std::min<int64_t>(4096, (n_pad + 7) / 8)), 256, 0, s>>>(
-            X, n, dim, n_pad, kp, terms, 0, cos, xb, xn, xx);
+        prep_rows<T><<<int(std::min<int64_t>(8192, (n_pad + 7) / 8)), 256, 0, s>>>(
+            X, n, dim, n_pad, kp, terms, 0, cos, xb, xn, xx, l2, INFINITY);
     XT(cudaGetLastError());
     launches++;
     double xmax = 1.0;  // largest data norm (margins): a device reduction, one 8-byte copy
@@ -1256,31 +1479,35 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
     CUtensorMap tmA, tmB;
     if (int rc = make_map(&tmA, B + o_qb, q_pad, kp, BM, bytes)) return rc;
     if (int rc = make_map(&tmB, B + o_xb, n_pad, kp, BN, bytes)) return rc;
-    const size_t smem = STAGES * STAGE_BYTES + XSLOTS * BN * 4 + 1024 + BAR_BYTES;
-    XT(cudaFuncSetAttribute(knn_filter_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    XT(cudaFuncSetAttribute(knn_filter_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    // Operand buffers: the query tile's operand resident beside at least three stages of rows where
+    // that fits, else loaded with every stage.
+    const int kchunks = kp / (bytes ? BK8 : BK);
+    const size_t room = SMEM_MAX - 1024 - XSLOTS * BN * 4 - BAR_BYTES;
+    const bool resident = size_t(kchunks) * A_BYTES + 3 * size_t(B_BYTES) <= room;
+    const size_t a_bytes = resident ? size_t(kchunks) * A_BYTES : 0;
+    const size_t stage_bytes = resident ? B_BYTES : A_BYTES + B_BYTES;
+    const int nstages = int(std::min<size_t>(MAX_STAGES, (room - a_bytes) / stage_bytes));
+    const size_t smem = a_bytes + nstages * stage_bytes + XSLOTS * BN * 4 + 1024 + BAR_BYTES;
     const int wpb = 4;
-    const size_t rsm = size_t(wpb) * (k + 1) * 12;
-    if (rsm > 200 * 1024) return fail(HNSW_B200_EINVAL, "k too large for the rerank kernel");
+    if (size_t(wpb) * (k + 1) * 12 > 200 * 1024) return fail(HNSW_B200_EINVAL, "k too large for the rerank kernel");
+    const bool products = !bytes && dim < COOP_DIM;
+    const bool gather = wpb * rerank_smem(k, dim, true, products) <= 200 * 1024;
+    const size_t rsm = wpb * rerank_smem(k, dim, gather, gather && products);
     XT(cudaFuncSetAttribute(rerank_topk<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(rsm)));
-    XT(cudaMemsetAsync(err, 0, 16, s));
-    auto *ferr = reinterpret_cast<unsigned long long *>(B + o_fe);  // measured filter error (bits)
-    XT(cudaMemsetAsync(ferr, 0, 8, s));
-    std::vector<float> inf(static_cast<size_t>(QB), INFINITY);
-    auto *cstat = reinterpret_cast<unsigned long long *>(B + o_cs);  // largest and total count
-    double max_margin = 0.0;
+    XT(cudaMemsetAsync(st, 0, sizeof(Stats), s));
+    Stats hst;
     int64_t total_cand = 0;
 
     for (int64_t q0 = 0; q0 < nq_all; q0 += QB) {
         const int64_t nq = std::min<int64_t>(QB, nq_all - q0);
         const T *Q = static_cast<const T *>(a->queries) + q0 * dim;
         if (bytes) {  // exact filter values: no margin
-            prep_rows_u8<T><<<int(std::min<int64_t>(4096, (q_pad + 7) / 8)), 256, 0, s>>>(
-                Q, nq, dim, q_pad, kp, qb8, qqi);
+            prep_rows_u8<T><<<int(std::min<int64_t>(4096, (q_pad + 31) / 32)), 256, 0, s>>>(
+                Q, nq, dim, q_pad, kp, qb8, qqi, vec(Q), l2, 0);
             XT(cudaMemsetAsync(mg, 0, size_t(nq) * 4, s));
         } else {
             prep_rows<T><<<int(std::min<int64_t>(4096, (q_pad + 7) / 8)), 256, 0, s>>>(
-                Q, nq, dim, q_pad, kp, terms, 1, cos, qb, qn, qq);
+                Q, nq, dim, q_pad, kp, terms, 1, cos, qb, qn, qq, l2, 0.f);
             margins_kernel<<<int((nq + 255) / 256), 256, 0, s>>>(qn, int32_t(nq), xmax, kp, terms, metric, mg);
         }
         XT(cudaGetLastError());
@@ -1288,107 +1515,97 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
         // Query tiles of this chunk only (the last chunk may be short), rows split to fill the GPU.
         const int qt_chunk = int((nq + BM - 1) / BM);
         int nseg = 0;  // segments per query of the last pass run
-        auto run_filter = [&](int64_t row_end, bool bmin) -> int {
-            const Geo gg = geo(nq, row_end);
-            const int tps = gg.tps, splits = gg.splits;
-            nseg = splits * EPI_PER_QUARTER;
+        auto run_filter = [&](int pass_tiles, int pass_stride, const float *pass_thr, bool bmin) -> int {
+            const Geo gg = geo(nq, pass_tiles);
+            nseg = gg.splits * EPI_PER_QUARTER;
             FilterParams fp;
             fp.nq = int32_t(nq);
-            fp.row_begin = 0;
-            fp.row_end = int32_t(row_end);
-            fp.kchunks = kp / (bytes ? BK8 : BK);
-            fp.tiles_per_split = tps;
+            fp.row_end = int32_t(n);
+            fp.tiles = pass_tiles;
+            fp.tile_stride = pass_stride;
+            fp.kchunks = kchunks;
+            fp.stages = nstages;
+            fp.a_resident = resident ? 1 : 0;
+            fp.tiles_per_split = gg.tps;
             fp.metric = metric;
             fp.qq = qq;
             fp.xx = xx;
             fp.qqi = qqi;
             fp.xxi = xxi;
-            fp.thr = th;
+            fp.thr = pass_thr;
             fp.cand_val = cv;
             fp.cand_id = ci;
             fp.cand_cnt = cnt;
             fp.cap = int32_t(cap);
-            fp.block_min = bmin ? 1 : 0;
-            fp.err = err;
-            if (bytes)
-                knn_filter_kernel<true><<<dim3(qt_chunk, splits), FILTER_THREADS, smem, s>>>(tmA, tmB, fp);
-            else
-                knn_filter_kernel<false><<<dim3(qt_chunk, splits), FILTER_THREADS, smem, s>>>(tmA, tmB, fp);
-            XT(cudaGetLastError());
+            fp.mul = metric == HNSW_B200_L2 ? -2 : -1;
+            fp.err = &st->err;
+            auto launch = [&](auto kern) -> int {
+                XT(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
+                kern<<<dim3(qt_chunk, gg.splits), FILTER_THREADS, smem, s>>>(tmA, tmB, fp);
+                XT(cudaGetLastError());
+                return 0;
+            };
+            const int rc = bytes ? (bmin ? launch(knn_filter_kernel<true, true>) : launch(knn_filter_kernel<true, false>))
+                                 : (bmin ? launch(knn_filter_kernel<false, true>) : launch(knn_filter_kernel<false, false>));
+            if (rc) return rc;
             launches++;
             return 0;
         };
-        // Pass one: the prefix rows with no threshold give tau (an upper bound of the k-th).
-        XT(cudaMemcpyAsync(th, inf.data(), size_t(nq) * 4, cudaMemcpyHostToDevice, s));
-        // One candidate per CW-row block suffices while the prefix has at least k blocks.
-        if (int rc = run_filter(prefix, block_min)) return rc;
-        // tau: the k-th smallest block minimum (a warp per query over its compacted list; a block
-        // per query over the segments measured 11% slower on the 60K x 784 set).
-        select_kth<<<int((nq + SELECT_WARPS - 1) / SELECT_WARPS), 32 * SELECT_WARPS, 0, s>>>(
-            cv, nullptr, cnt, int32_t(cap), int32_t(nseg), int32_t(nq), k, mg, th, tau, cm);
-        // Pass two: every row against tau + margin.
-        if (int rc = run_filter(n, false)) return rc;
-        XT(cudaMemsetAsync(cstat, 0, 16, s));
-        count_stats<<<int(std::min<int64_t>(1024, (nq * nseg + 255) / 256)), 256, 0, s>>>(
-            cnt, nq * nseg, cstat);
-        XT(cudaGetLastError());
-        launches++;
-        int32_t herr[4];
-        unsigned long long hst[2];
-        XT(cudaMemcpyAsync(hst, cstat, 16, cudaMemcpyDeviceToHost, s));
-        XT(cudaMemcpyAsync(herr, err, 16, cudaMemcpyDeviceToHost, s));
-        XT(cudaStreamSynchronize(s));
-        if (herr[0]) return fail(HNSW_B200_ECUDA, "exact knn: a bounded wait expired in the filter kernel");
-        const int64_t worst = int64_t(hst[0]);
-        total_cand += int64_t(hst[1]);
-        if (worst > cap) {
-            *cap_needed = worst;
-            return fail(HNSW_B200_ERETRY, "exact knn: candidate buffer overflow (" + std::to_string(worst) +
-                                              " > " + std::to_string(cap) + ")");
-        }
-        // The k-th smallest candidate is the global k-th approximate distance: final threshold.
-        select_kth<<<int((nq + SELECT_WARPS - 1) / SELECT_WARPS), 32 * SELECT_WARPS, 0, s>>>(
-            cv, ci, cnt, int32_t(cap), int32_t(nseg), int32_t(nq), k, mg, th, tau, cm);
-        rerank_topk<T><<<int((nq + wpb - 1) / wpb), wpb * 32, rsm, s>>>(
-            X, Q, dim, int32_t(nq), k, metric, xn, qn, cv, ci, cm, int32_t(cap), int32_t(nseg), th,
-            a->out_ids + q0 * k, a->out_dists + q0 * k, ferr, bytes ? EXACT_LIM : 0.f, err + 1);
-        XT(cudaGetLastError());
-        launches += 3;
-        if (a->out_filter_error_bound) {
-            // BF16 filter: half the largest margin. Byte rows: the integer distances are exact and
-            // only their float copies of 2^24 or more round, by at most half a float ulp of the
-            // final threshold (counted here as a margin of a whole ulp).
-            std::vector<float> hm(static_cast<size_t>(nq));
-            XT(cudaMemcpyAsync(hm.data(), bytes ? th : mg, size_t(nq) * 4, cudaMemcpyDeviceToHost, s));
+        for (int pass_rank = rank;; pass_rank = k) {
+            // Pass one: the sampled tiles give tau, the threshold of pass two.
+            if (int rc = run_filter(sample, stride, nullptr, block_min)) return rc;
+            const int sel_blocks = int((nq + SELECT_WARPS - 1) / SELECT_WARPS);
+            select_kth<<<sel_blocks, 32 * SELECT_WARPS, 0, s>>>(
+                cv, nullptr, cnt, int32_t(cap), int32_t(nseg), int32_t(nq), pass_rank, mg, th, tau, cm, 0,
+                bytes, nullptr, nullptr);
+            // Pass two: every row against tau + margin; the k-th smallest candidate is the global
+            // k-th approximate distance, the final threshold.
+            if (int rc = run_filter(tiles, 1, th, false)) return rc;
+            count_stats<<<int(std::min<int64_t>(1024, (nq * nseg + 255) / 256)), 256, 0, s>>>(
+                cnt, nq * nseg, &st->longest);
+            select_kth<<<sel_blocks, 32 * SELECT_WARPS, 0, s>>>(
+                cv, ci, cnt, int32_t(cap), int32_t(nseg), int32_t(nq), k, mg, th, tau, cm, 1, bytes,
+                &st->short_lists, &st->bound);
+            rerank_topk<T><<<int((nq + wpb - 1) / wpb), wpb * 32, rsm, s>>>(
+                X, Q, dim, int32_t(nq), k, metric, xn, qn, cv, ci, cm, int32_t(cap), int32_t(nseg), th,
+                a->out_ids + q0 * k, a->out_dists + q0 * k, &st->filter_err, bytes ? EXACT_LIM : 0.f,
+                &st->mismatch, gather, gather && products);
+            XT(cudaGetLastError());
+            launches += 4;
+            XT(cudaMemcpyAsync(&hst, st, sizeof(Stats), cudaMemcpyDeviceToHost, s));
+            XT(cudaMemsetAsync(st, 0, offsetof(Stats, filter_err), s));
             XT(cudaStreamSynchronize(s));
-            for (float v : hm) {
-                // inner product: candidates reach below the threshold, down to -dim 255^2
-                if (bytes && metric == HNSW_B200_IP) v = float(dim) * 65025.f;
-                if (!bytes) {
-                    max_margin = std::max(max_margin, double(v));
-                } else if (std::fabs(v) >= EXACT_LIM && std::isfinite(v)) {
-                    int e = 0;
-                    std::frexp(double(std::fabs(v)), &e);  // |v| in [2^(e-1), 2^e)
-                    max_margin = std::max(max_margin, std::ldexp(1.0, e - 24));
-                }
+            if (hst.err) return fail(HNSW_B200_ECUDA, "exact knn: a bounded wait expired in the filter kernel");
+            if (int64_t(hst.longest) > cap) {
+                *cap_needed = int64_t(hst.longest);
+                return fail(HNSW_B200_ERETRY, "exact knn: candidate buffer overflow (" +
+                                                  std::to_string(hst.longest) + " > " + std::to_string(cap) + ")");
             }
+            if (!hst.short_lists || pass_rank == k) break;
         }
+        if (bytes && hst.mismatch)  // the integer results against their float64 re-scores
+            return fail(HNSW_B200_ECUDA, "exact knn: an integer filter distance differs from its float64 re-score");
+        total_cand += int64_t(hst.total);
     }
-    if (bytes) {  // the integer results against their float64 re-scores
-        int32_t hm[4];
-        XT(cudaMemcpyAsync(hm, err, 16, cudaMemcpyDeviceToHost, s));
-        XT(cudaStreamSynchronize(s));
-        if (hm[1]) return fail(HNSW_B200_ECUDA, "exact knn: an integer filter distance differs from its float64 re-score");
+    if (a->out_filter_error_bound) {
+        // BF16 filter: half the largest margin. Byte rows: the integer distances are exact and
+        // only their float copies of 2^24 or more round, by at most half a float ulp of the
+        // final threshold (counted here as a margin of a whole ulp).
+        float v;
+        std::memcpy(&v, &hst.bound, 4);
+        // inner product: candidates reach below the threshold, down to -dim 255^2
+        if (bytes && metric == HNSW_B200_IP) v = float(dim) * 65025.f;
+        double max_margin = 0.0;
+        if (!bytes) {
+            max_margin = double(v);
+        } else if (v >= EXACT_LIM) {
+            int e = 0;
+            std::frexp(double(v), &e);  // v in [2^(e-1), 2^e)
+            max_margin = std::ldexp(1.0, e - 24);
+        }
+        *a->out_filter_error_bound = max_margin / 2.0;
     }
-    if (a->out_filter_error_bound) *a->out_filter_error_bound = max_margin / 2.0;
-    if (a->out_filter_max_error) {
-        unsigned long long bits = 0;
-        XT(cudaMemcpyAsync(&bits, ferr, 8, cudaMemcpyDeviceToHost, s));
-        XT(cudaStreamSynchronize(s));
-        double e = 0.0;
-        std::memcpy(&e, &bits, 8);
-        *a->out_filter_max_error = e;
-    }
+    if (a->out_filter_max_error) std::memcpy(a->out_filter_max_error, &hst.filter_err, 8);
     if (a->out_candidates) *a->out_candidates = total_cand;
     if (a->out_launches) *a->out_launches = launches;
     return 0;
