@@ -85,86 +85,128 @@ __device__ __forceinline__ float forward(const float *s, const float *x, int lan
     return o + b3[0];
 }
 
-// Per-sample forward and backward: activations and their gradients for the reduction kernel.
-__global__ void mlp_fwd_bwd(const float *P, const float *X, const float *Y, int B, float *H1,
-                            float *H2, float *dH1, float *dH2, float *dO, float *loss) {
-    extern __shared__ float sw[];
+// Samples of a block's tile: their activations and gradients stay in shared memory.
+constexpr int TS = 32;
+constexpr int GRAD_THREADS = 512;  // 16 warps, two samples of a tile each
+constexpr int MAX_ROWS = 296;      // blocks (rows of partial sums): two a SM
+constexpr int GRAD_FLOATS = (SMEM_FLOATS + 3) / 4 * 4 + 4 * TS * H + TS * F + TS;
+
+// Forward, backward and weight gradients of the batch: block r writes row r of part (NPARAM partial sums).
+// A tile of 32 samples is run through the network a warp a sample; then every thread adds the tile's
+// products to the parameters it owns (W2: 4 x 2 of its elements, read from shared memory as one 16-byte
+// broadcast and one 8-byte load a sample; W1, W3, biases: up to three single ones), tile after tile in
+// order, so the sums are deterministic. Bound by the shuffles and shared-memory reads of the passes,
+// about 900 instructions a sample. (Writing the activations out and adding the whole batch up in
+// one thread a parameter took 15 + 182 us a step of 4,096 samples; this kernel takes 20, mlp_finish 4.)
+__global__ void __launch_bounds__(GRAD_THREADS) mlp_grad_tiles(const float *P, const float *X, const float *Y,
+                                                               int B, float *part, float *loss) {
+    extern __shared__ __align__(16) float sw[];
+    float *h1 = sw + (SMEM_FLOATS + 3) / 4 * 4, *h2 = h1 + TS * H, *d1 = h2 + TS * H, *d2 = d1 + TS * H;
+    float *xs = d2 + TS * H, *dos = xs + TS * F;
     load_weights(P, sw);
     const float *w2 = sw + H * S_W1 + H, *w3 = w2 + H * S_W2 + H;
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    float lsum = 0.f;
-    for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < B; b += warps) {
-        float x[F];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int j0 = (t >> 5) * 4, i0 = (t & 31) * 2;  // W2[j0 .. j0 + 3][i0 .. i0 + 1]
+    const int p1 = t, p1b = t + GRAD_THREADS;          // W1 elements
+    float aw2[4][2] = {}, aw1 = 0.f, aw1b = 0.f, arest = 0.f, lsum = 0.f;
+    const int tiles = (B + TS - 1) / TS;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int b0 = tile * TS, nb = min(TS, B - b0);
+        for (int s = warp; s < nb; s += GRAD_THREADS / 32) {
+            const int b = b0 + s;
+            float x[F];
 #pragma unroll
-        for (int i = 0; i < F; i++) x[i] = X[int64_t(b) * F + i];
-        float h1a, h1b, h2a, h2b;
-        const float o = forward(sw, x, lane, h1a, h1b, h2a, h2b);
-        const float err = o - Y[b];
-        const float g = 2.f * err / float(B);
-        lsum += err * err / float(B);
-        const float g2a = h2a > 0.f ? g * w3[lane] : 0.f;
-        const float g2b = h2b > 0.f ? g * w3[lane + 32] : 0.f;
-        // dh1[i] = sum_j W2[j][i] dh2[j]; lane i holds i and i + 32.
-        float g1a = 0.f, g1b = 0.f;
+            for (int i = 0; i < F; i++) x[i] = X[int64_t(b) * F + i];
+            float h1a, h1b, h2a, h2b;
+            const float o = forward(sw, x, lane, h1a, h1b, h2a, h2b);
+            const float err = o - Y[b];
+            const float g = 2.f * err / float(B);
+            lsum += err * err / float(B);
+            const float g2a = h2a > 0.f ? g * w3[lane] : 0.f;
+            const float g2b = h2b > 0.f ? g * w3[lane + 32] : 0.f;
+            // dh1[i] = sum_j W2[j][i] dh2[j]; lane i holds i and i + 32.
+            float g1a = 0.f, g1b = 0.f;
 #pragma unroll 8
-        for (int j = 0; j < 32; j++) {
-            const float u = __shfl_sync(FULL, g2a, j), v = __shfl_sync(FULL, g2b, j);
-            g1a = fmaf(w2[j * S_W2 + lane], u, g1a);
-            g1b = fmaf(w2[j * S_W2 + lane + 32], u, g1b);
-            g1a = fmaf(w2[(j + 32) * S_W2 + lane], v, g1a);
-            g1b = fmaf(w2[(j + 32) * S_W2 + lane + 32], v, g1b);
+            for (int j = 0; j < 32; j++) {
+                const float u = __shfl_sync(FULL, g2a, j), v = __shfl_sync(FULL, g2b, j);
+                g1a = fmaf(w2[j * S_W2 + lane], u, g1a);
+                g1b = fmaf(w2[j * S_W2 + lane + 32], u, g1b);
+                g1a = fmaf(w2[(j + 32) * S_W2 + lane], v, g1a);
+                g1b = fmaf(w2[(j + 32) * S_W2 + lane + 32], v, g1b);
+            }
+            h1[s * H + lane] = h1a;
+            h1[s * H + lane + 32] = h1b;
+            h2[s * H + lane] = h2a;
+            h2[s * H + lane + 32] = h2b;
+            d1[s * H + lane] = h1a > 0.f ? g1a : 0.f;
+            d1[s * H + lane + 32] = h1b > 0.f ? g1b : 0.f;
+            d2[s * H + lane] = g2a;
+            d2[s * H + lane + 32] = g2b;
+            if (lane < F) xs[s * F + lane] = X[int64_t(b) * F + lane];
+            if (lane == 0) dos[s] = g;
         }
-        g1a = h1a > 0.f ? g1a : 0.f;
-        g1b = h1b > 0.f ? g1b : 0.f;
-        const int64_t r = int64_t(b) * H;
-        H1[r + lane] = h1a;
-        H1[r + lane + 32] = h1b;
-        H2[r + lane] = h2a;
-        H2[r + lane + 32] = h2b;
-        dH1[r + lane] = g1a;
-        dH1[r + lane + 32] = g1b;
-        dH2[r + lane] = g2a;
-        dH2[r + lane + 32] = g2b;
-        if (lane == 0) dO[b] = g;
+        __syncthreads();
+        // dW1 = dH1^T X, dW2 = dH2^T H1, dW3 = dO^T H2, biases the column sums
+#pragma unroll 4
+        for (int s = 0; s < nb; s++) {
+            const float4 d = *reinterpret_cast<const float4 *>(d2 + s * H + j0);
+            const float2 h = *reinterpret_cast<const float2 *>(h1 + s * H + i0);
+            aw2[0][0] = fmaf(d.x, h.x, aw2[0][0]);
+            aw2[0][1] = fmaf(d.x, h.y, aw2[0][1]);
+            aw2[1][0] = fmaf(d.y, h.x, aw2[1][0]);
+            aw2[1][1] = fmaf(d.y, h.y, aw2[1][1]);
+            aw2[2][0] = fmaf(d.z, h.x, aw2[2][0]);
+            aw2[2][1] = fmaf(d.z, h.y, aw2[2][1]);
+            aw2[3][0] = fmaf(d.w, h.x, aw2[3][0]);
+            aw2[3][1] = fmaf(d.w, h.y, aw2[3][1]);
+        }
+        for (int s = 0; s < nb; s++) {
+            aw1 = fmaf(d1[s * H + p1 / F], xs[s * F + p1 % F], aw1);
+            if (p1b < H * F) aw1b = fmaf(d1[s * H + p1b / F], xs[s * F + p1b % F], aw1b);
+            if (t < H) arest += d1[s * H + t];
+            else if (t < 2 * H) arest += d2[s * H + t - H];
+            else if (t < 3 * H) arest = fmaf(dos[s], h2[s * H + t - 2 * H], arest);
+            else if (t == 3 * H) arest += dos[s];
+        }
+        __syncthreads();  // before the next tile's samples are written
     }
+    float *row = part + int64_t(blockIdx.x) * NPARAM;
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+        row[O_W2 + (j0 + a) * H + i0] = aw2[a][0];
+        row[O_W2 + (j0 + a) * H + i0 + 1] = aw2[a][1];
+    }
+    row[O_W1 + p1] = aw1;
+    if (p1b < H * F) row[O_W1 + p1b] = aw1b;
+    if (t < H) row[O_B1 + t] = arest;
+    else if (t < 2 * H) row[O_B2 + t - H] = arest;
+    else if (t < 3 * H) row[O_W3 + t - 2 * H] = arest;
+    else if (t == 3 * H) row[O_B3] = arest;
     if (lane == 0 && lsum != 0.f) atomicAdd(loss, lsum);
 }
 
-// Weight gradients: one thread per parameter, summed over the batch in a fixed order
-// (deterministic). dW1 = dH1^T X, dW2 = dH2^T H1, dW3 = dO^T H2, biases the column sums.
-__global__ void mlp_grads(const float *X, const float *H1, const float *H2, const float *dH1,
-                          const float *dH2, const float *dO, int B, float *G) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= NPARAM) return;
+// A parameter's gradient: the rows of partial sums added up in a fixed order, four threads a parameter
+// (rows 0, 4, 8, ...; 1, 5, ...; then the four sums). G != NULL: written there. Else one Adam step
+// (Kingma & Ba) with bias correction on the float32 masters.
+constexpr int FIN_PARAMS = 64;
+__global__ void mlp_finish(const float *part, int rows, float *G, float *P, float *M, float *V, float lr, float b1,
+                           float b2, float eps, float c1, float c2) {
+    __shared__ float sums[4][FIN_PARAMS];
+    const int i = threadIdx.x % FIN_PARAMS, q = threadIdx.x / FIN_PARAMS;
+    const int p = blockIdx.x * FIN_PARAMS + i;
     float acc = 0.f;
-    if (p < O_B1) {
-        const int j = p / F, i = p % F;
-        for (int b = 0; b < B; b++) acc = fmaf(dH1[int64_t(b) * H + j], X[int64_t(b) * F + i], acc);
-    } else if (p < O_W2) {
-        const int j = p - O_B1;
-        for (int b = 0; b < B; b++) acc += dH1[int64_t(b) * H + j];
-    } else if (p < O_B2) {
-        const int j = (p - O_W2) / H, i = (p - O_W2) % H;
-        for (int b = 0; b < B; b++) acc = fmaf(dH2[int64_t(b) * H + j], H1[int64_t(b) * H + i], acc);
-    } else if (p < O_W3) {
-        const int j = p - O_B2;
-        for (int b = 0; b < B; b++) acc += dH2[int64_t(b) * H + j];
-    } else if (p < O_B3) {
-        const int j = p - O_W3;
-        for (int b = 0; b < B; b++) acc = fmaf(dO[b], H2[int64_t(b) * H + j], acc);
-    } else {
-        for (int b = 0; b < B; b++) acc += dO[b];
+    if (p < NPARAM) {
+#pragma unroll 8
+        for (int r = q; r < rows; r += 4) acc += part[int64_t(r) * NPARAM + p];
     }
-    G[p] = acc;
-}
-
-// Adam (Kingma & Ba) with bias correction, on the float32 masters.
-__global__ void mlp_adam(float *P, const float *G, float *M, float *V, int n, float lr, float b1,
-                         float b2, float eps, float c1, float c2) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const float g = G[p];
+    sums[q][i] = acc;
+    __syncthreads();
+    if (q != 0 || p >= NPARAM) return;
+    const float g = (sums[0][i] + sums[1][i]) + (sums[2][i] + sums[3][i]);
+    if (G) {
+        G[p] = g;
+        return;
+    }
     const float m = b1 * M[p] + (1.f - b1) * g;
     const float v = b2 * V[p] + (1.f - b2) * g * g;
     M[p] = m;
@@ -215,7 +257,18 @@ __global__ void mlp_pack_kernel(const float *P, const float *mean, const float *
     }
 }
 
-size_t scratch_floats(int B) { return size_t(B) * (4 * H + 1) + NPARAM + 4; }
+size_t scratch_floats(int B) { return size_t(B) * (4 * H + 1) + NPARAM + 4; }  // at least the partial sums
+
+// Launches the batch's gradients into rows of part (scratch), and returns how many rows.
+int grad_rows(const float *params, const float *features, const float *targets, int batch, float *part,
+              float *loss, cudaStream_t s) {
+    const int rows = std::min(MAX_ROWS, (batch + TS - 1) / TS);
+    cudaFuncSetAttribute(mlp_grad_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, GRAD_FLOATS * 4);
+    cudaMemsetAsync(loss, 0, sizeof(float), s);
+    mlp_grad_tiles<<<rows, GRAD_THREADS, GRAD_FLOATS * sizeof(float), s>>>(params, features, targets, batch, part,
+                                                                            loss);
+    return rows;
+}
 
 }  // namespace hbm
 
@@ -240,18 +293,11 @@ int hnsw_b200_mlp_train_step(float *params, float *adam_m, float *adam_v, int64_
         step < 1)
         return hb::fail(HNSW_B200_EINVAL, "mlp_train_step: bad argument");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    float *H1 = scratch, *H2 = H1 + size_t(batch) * H, *dH1 = H2 + size_t(batch) * H;
-    float *dH2 = dH1 + size_t(batch) * H, *dO = dH2 + size_t(batch) * H, *G = dO + batch;
-    const int threads = 256;
-    const int blocks = std::min(1184, (batch * 32 + threads - 1) / threads);
-    cudaMemsetAsync(loss, 0, sizeof(float), s);
-    mlp_fwd_bwd<<<blocks, threads, SMEM_FLOATS * sizeof(float), s>>>(params, features, targets,
-                                                                       batch, H1, H2, dH1, dH2, dO, loss);
-    mlp_grads<<<(NPARAM + 127) / 128, 128, 0, s>>>(features, H1, H2, dH1, dH2, dO, batch, G);
+    const int rows = grad_rows(params, features, targets, batch, scratch, loss, s);
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - powf(b1, float(step)), c2 = 1.f - powf(b2, float(step));
-    mlp_adam<<<(NPARAM + 255) / 256, 256, 0, s>>>(params, G, adam_m, adam_v, NPARAM, lr, b1, b2,
-                                                  1e-8f, c1, c2);
+    mlp_finish<<<(NPARAM + FIN_PARAMS - 1) / FIN_PARAMS, 4 * FIN_PARAMS, 0, s>>>(
+        scratch, rows, nullptr, params, adam_m, adam_v, lr, b1, b2, 1e-8f, c1, c2);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return hb::fail(HNSW_B200_ECUDA, std::string("mlp train: ") + cudaGetErrorString(e));
     return 0;
@@ -264,14 +310,9 @@ int hnsw_b200_mlp_gradients(const float *params, const float *features, const fl
     if (!params || !features || !targets || !scratch || !grads || !loss || batch < 1)
         return hb::fail(HNSW_B200_EINVAL, "mlp_gradients: bad argument");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    float *H1 = scratch, *H2 = H1 + size_t(batch) * H, *dH1 = H2 + size_t(batch) * H;
-    float *dH2 = dH1 + size_t(batch) * H, *dO = dH2 + size_t(batch) * H;
-    const int threads = 256;
-    const int blocks = std::min(1184, (batch * 32 + threads - 1) / threads);
-    cudaMemsetAsync(loss, 0, sizeof(float), s);
-    mlp_fwd_bwd<<<blocks, threads, SMEM_FLOATS * sizeof(float), s>>>(params, features, targets,
-                                                                       batch, H1, H2, dH1, dH2, dO, loss);
-    mlp_grads<<<(NPARAM + 127) / 128, 128, 0, s>>>(features, H1, H2, dH1, dH2, dO, batch, grads);
+    const int rows = grad_rows(params, features, targets, batch, scratch, loss, s);
+    mlp_finish<<<(NPARAM + FIN_PARAMS - 1) / FIN_PARAMS, 4 * FIN_PARAMS, 0, s>>>(
+        scratch, rows, grads, nullptr, nullptr, nullptr, 0.f, 0.f, 0.f, 0.f, 1.f, 1.f);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return hb::fail(HNSW_B200_ECUDA, std::string("mlp grads: ") + cudaGetErrorString(e));
     return 0;
