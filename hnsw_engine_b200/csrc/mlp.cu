@@ -85,133 +85,195 @@ __device__ __forceinline__ float forward(const float *s, const float *x, int lan
     return o + b3[0];
 }
 
-// Samples of a block's tile: their activations and gradients stay in shared memory.
-constexpr int TS = 32;
-constexpr int GRAD_THREADS = 512;  // 16 warps, two samples of a tile each
-constexpr int MAX_ROWS = 296;      // blocks (rows of partial sums): two a SM
-constexpr int GRAD_FLOATS = (SMEM_FLOATS + 3) / 4 * 4 + 4 * TS * H + TS * F + TS;
-
-// Forward, backward and weight gradients of the batch: block r writes row r of part (NPARAM partial sums).
-// A tile of 32 samples is run through the network a warp a sample; then every thread adds the tile's
-// products to the parameters it owns (W2: 4 x 2 of its elements, read from shared memory as one 16-byte
-// broadcast and one 8-byte load a sample; W1, W3, biases: up to three single ones), tile after tile in
-// order, so the sums are deterministic. Bound by the shuffles and shared-memory reads of the passes,
-// about 900 instructions a sample. (Writing the activations out and adding the whole batch up in
-// one thread a parameter took 15 + 182 us a step of 4,096 samples; this kernel takes 20, mlp_finish 4.)
-__global__ void __launch_bounds__(GRAD_THREADS) mlp_grad_tiles(const float *P, const float *X, const float *Y,
-                                                               int B, float *part, float *loss) {
-    extern __shared__ __align__(16) float sw[];
-    float *h1 = sw + (SMEM_FLOATS + 3) / 4 * 4, *h2 = h1 + TS * H, *d1 = h2 + TS * H, *d2 = d1 + TS * H;
-    float *xs = d2 + TS * H, *dos = xs + TS * F;
+// Per-sample forward and backward: activations and their gradients for the reduction kernel.
+__global__ void mlp_fwd_bwd(const float *P, const float *X, const float *Y, int B, float *H1,
+                            float *H2, float *dH1, float *dH2, float *dO, float *loss) {
+    extern __shared__ float sw[];
     load_weights(P, sw);
     const float *w2 = sw + H * S_W1 + H, *w3 = w2 + H * S_W2 + H;
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int j0 = (t >> 5) * 4, i0 = (t & 31) * 2;  // W2[j0 .. j0 + 3][i0 .. i0 + 1]
-    const int p1 = t, p1b = t + GRAD_THREADS;          // W1 elements
-    float aw2[4][2] = {}, aw1 = 0.f, aw1b = 0.f, arest = 0.f, lsum = 0.f;
-    const int tiles = (B + TS - 1) / TS;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int b0 = tile * TS, nb = min(TS, B - b0);
-        for (int s = warp; s < nb; s += GRAD_THREADS / 32) {
-            const int b = b0 + s;
-            float x[F];
+    const int lane = threadIdx.x & 31;
+    const int warps = (gridDim.x * blockDim.x) >> 5;
+    float lsum = 0.f;
+    for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < B; b += warps) {
+        float x[F];
 #pragma unroll
-            for (int i = 0; i < F; i++) x[i] = X[int64_t(b) * F + i];
-            float h1a, h1b, h2a, h2b;
-            const float o = forward(sw, x, lane, h1a, h1b, h2a, h2b);
-            const float err = o - Y[b];
-            const float g = 2.f * err / float(B);
-            lsum += err * err / float(B);
-            const float g2a = h2a > 0.f ? g * w3[lane] : 0.f;
-            const float g2b = h2b > 0.f ? g * w3[lane + 32] : 0.f;
-            // dh1[i] = sum_j W2[j][i] dh2[j]; lane i holds i and i + 32.
-            float g1a = 0.f, g1b = 0.f;
+        for (int i = 0; i < F; i++) x[i] = X[int64_t(b) * F + i];
+        float h1a, h1b, h2a, h2b;
+        const float o = forward(sw, x, lane, h1a, h1b, h2a, h2b);
+        const float err = o - Y[b];
+        const float g = 2.f * err / float(B);
+        lsum += err * err / float(B);
+        const float g2a = h2a > 0.f ? g * w3[lane] : 0.f;
+        const float g2b = h2b > 0.f ? g * w3[lane + 32] : 0.f;
+        // dh1[i] = sum_j W2[j][i] dh2[j]; lane i holds i and i + 32.
+        float g1a = 0.f, g1b = 0.f;
 #pragma unroll 8
-            for (int j = 0; j < 32; j++) {
-                const float u = __shfl_sync(FULL, g2a, j), v = __shfl_sync(FULL, g2b, j);
-                g1a = fmaf(w2[j * S_W2 + lane], u, g1a);
-                g1b = fmaf(w2[j * S_W2 + lane + 32], u, g1b);
-                g1a = fmaf(w2[(j + 32) * S_W2 + lane], v, g1a);
-                g1b = fmaf(w2[(j + 32) * S_W2 + lane + 32], v, g1b);
-            }
-            h1[s * H + lane] = h1a;
-            h1[s * H + lane + 32] = h1b;
-            h2[s * H + lane] = h2a;
-            h2[s * H + lane + 32] = h2b;
-            d1[s * H + lane] = h1a > 0.f ? g1a : 0.f;
-            d1[s * H + lane + 32] = h1b > 0.f ? g1b : 0.f;
-            d2[s * H + lane] = g2a;
-            d2[s * H + lane + 32] = g2b;
-            if (lane < F) xs[s * F + lane] = X[int64_t(b) * F + lane];
-            if (lane == 0) dos[s] = g;
+        for (int j = 0; j < 32; j++) {
+            const float u = __shfl_sync(FULL, g2a, j), v = __shfl_sync(FULL, g2b, j);
+            g1a = fmaf(w2[j * S_W2 + lane], u, g1a);
+            g1b = fmaf(w2[j * S_W2 + lane + 32], u, g1b);
+            g1a = fmaf(w2[(j + 32) * S_W2 + lane], v, g1a);
+            g1b = fmaf(w2[(j + 32) * S_W2 + lane + 32], v, g1b);
         }
-        __syncthreads();
-        // dW1 = dH1^T X, dW2 = dH2^T H1, dW3 = dO^T H2, biases the column sums
-#pragma unroll 4
-        for (int s = 0; s < nb; s++) {
-            const float4 d = *reinterpret_cast<const float4 *>(d2 + s * H + j0);
-            const float2 h = *reinterpret_cast<const float2 *>(h1 + s * H + i0);
-            aw2[0][0] = fmaf(d.x, h.x, aw2[0][0]);
-            aw2[0][1] = fmaf(d.x, h.y, aw2[0][1]);
-            aw2[1][0] = fmaf(d.y, h.x, aw2[1][0]);
-            aw2[1][1] = fmaf(d.y, h.y, aw2[1][1]);
-            aw2[2][0] = fmaf(d.z, h.x, aw2[2][0]);
-            aw2[2][1] = fmaf(d.z, h.y, aw2[2][1]);
-            aw2[3][0] = fmaf(d.w, h.x, aw2[3][0]);
-            aw2[3][1] = fmaf(d.w, h.y, aw2[3][1]);
-        }
-        for (int s = 0; s < nb; s++) {
-            aw1 = fmaf(d1[s * H + p1 / F], xs[s * F + p1 % F], aw1);
-            if (p1b < H * F) aw1b = fmaf(d1[s * H + p1b / F], xs[s * F + p1b % F], aw1b);
-            if (t < H) arest += d1[s * H + t];
-            else if (t < 2 * H) arest += d2[s * H + t - H];
-            else if (t < 3 * H) arest = fmaf(dos[s], h2[s * H + t - 2 * H], arest);
-            else if (t == 3 * H) arest += dos[s];
-        }
-        __syncthreads();  // before the next tile's samples are written
+        g1a = h1a > 0.f ? g1a : 0.f;
+        g1b = h1b > 0.f ? g1b : 0.f;
+        const int64_t r = int64_t(b) * H;
+        H1[r + lane] = h1a;
+        H1[r + lane + 32] = h1b;
+        H2[r + lane] = h2a;
+        H2[r + lane + 32] = h2b;
+        dH1[r + lane] = g1a;
+        dH1[r + lane + 32] = g1b;
+        dH2[r + lane] = g2a;
+        dH2[r + lane + 32] = g2b;
+        if (lane == 0) dO[b] = g;
     }
-    float *row = part + int64_t(blockIdx.x) * NPARAM;
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-        row[O_W2 + (j0 + a) * H + i0] = aw2[a][0];
-        row[O_W2 + (j0 + a) * H + i0 + 1] = aw2[a][1];
-    }
-    row[O_W1 + p1] = aw1;
-    if (p1b < H * F) row[O_W1 + p1b] = aw1b;
-    if (t < H) row[O_B1 + t] = arest;
-    else if (t < 2 * H) row[O_B2 + t - H] = arest;
-    else if (t < 3 * H) row[O_W3 + t - 2 * H] = arest;
-    else if (t == 3 * H) row[O_B3] = arest;
     if (lane == 0 && lsum != 0.f) atomicAdd(loss, lsum);
 }
 
-// A parameter's gradient: the rows of partial sums added up in a fixed order, four threads a parameter
-// (rows 0, 4, 8, ...; 1, 5, ...; then the four sums). G != NULL: written there. Else one Adam step
-// (Kingma & Ba) with bias correction on the float32 masters.
-constexpr int FIN_PARAMS = 64;
-__global__ void mlp_finish(const float *part, int rows, float *G, float *P, float *M, float *V, float lr, float b1,
-                           float b2, float eps, float c1, float c2) {
-    __shared__ float sums[4][FIN_PARAMS];
-    const int i = threadIdx.x % FIN_PARAMS, q = threadIdx.x / FIN_PARAMS;
-    const int p = blockIdx.x * FIN_PARAMS + i;
-    float acc = 0.f;
-    if (p < NPARAM) {
-#pragma unroll 8
-        for (int r = q; r < rows; r += 4) acc += part[int64_t(r) * NPARAM + p];
+// Weight gradients dW1 = dH1^T X, dW2 = dH2^T H1, dW3 = dO^T H2, biases the column sums: every parameter
+// is summed over the batch by one thread, sample after sample (deterministic, and the order in which the
+// shipped networks were trained). What bounds that is the chain of one fused multiply-add a sample,
+// four cycles each, so the samples must be at hand: a block owns parameters that share columns, copies
+// those columns of 64 samples at a time into shared memory with cp.async, GRAD_STAGES - 1 chunks ahead, by
+// four warps of its own (one warp a scheduler adds, and would not hide the copies' instructions either). With each thread loading from memory as it went, a batch of 4,096
+// took 182 us; this takes 35, the Adam step included.
+//  blocks 0..15: W2 rows 4 r .. 4 r + 3, two a thread (H1 whole, four columns of dH2);
+//  16..21: W1 columns 2 r, 2 r + 1 (dH1 whole, X);  22: b1;  23: b2;  24: W3 and b3 (H2 whole, dO).
+// G != NULL: the gradients are written there. Else one Adam step (Kingma & Ba) with bias correction on the
+// float32 masters.
+constexpr int GRAD_CHUNK = 64, GRAD_STAGES = 4, ADD_THREADS = 128, GRAD_THREADS = 256, GRAD_BLOCKS = 25;
+constexpr int COPY_THREADS = GRAD_THREADS - ADD_THREADS;
+constexpr int GRAD_S2 = 16;  // floats a sample of the second array: 4 (dH2), 12 (X) or 1 (dO)
+constexpr int GRAD_STAGE_FLOATS = GRAD_CHUNK * (H + GRAD_S2);
+
+struct AdamArgs {
+    float *P, *M, *V;
+    float lr, b1, b2, eps, c1, c2;
+};
+
+__device__ __forceinline__ void copy_async(float *dst, const float *src, bool by16) {
+    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+    if (by16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+}
+
+// count contiguous floats, by the copying threads
+__device__ __forceinline__ void copy_run(float *dst, const float *src, int count, bool by16) {
+    const int t = threadIdx.x - ADD_THREADS, n4 = by16 ? count >> 2 : 0;
+    for (int e = t; e < n4; e += COPY_THREADS) copy_async(dst + 4 * e, src + 4 * e, true);
+    for (int e = 4 * n4 + t; e < count; e += COPY_THREADS) copy_async(dst + e, src + e, false);
+}
+
+// add(load(b)) for the nb samples of a chunk, in order. A whole chunk goes 16 samples at a time, the next
+// 16 read from shared memory while the multiply-adds of the current ones run (one warp a scheduler: nothing
+// else hides the reads).
+template <class Load, class Add>
+__device__ __forceinline__ void each_sample(int nb, Load load, Add add) {
+    if (nb == GRAD_CHUNK) {
+        constexpr int R = 16;
+        decltype(load(0)) v[2][R];
+#pragma unroll
+        for (int i = 0; i < R; i++) v[0][i] = load(i);
+#pragma unroll
+        for (int k = 0; k < GRAD_CHUNK / R; k++) {
+            if (k + 1 < GRAD_CHUNK / R) {
+#pragma unroll
+                for (int i = 0; i < R; i++) v[(k + 1) & 1][i] = load((k + 1) * R + i);
+            }
+#pragma unroll
+            for (int i = 0; i < R; i++) add(v[k & 1][i]);
+        }
+    } else {
+        for (int b = 0; b < nb; b++) add(load(b));
     }
-    sums[q][i] = acc;
-    __syncthreads();
-    if (q != 0 || p >= NPARAM) return;
-    const float g = (sums[0][i] + sums[1][i]) + (sums[2][i] + sums[3][i]);
-    if (G) {
-        G[p] = g;
-        return;
+}
+
+__global__ void __launch_bounds__(GRAD_THREADS) mlp_grads(const float *X, const float *H1, const float *H2,
+                                                          const float *dH1, const float *dH2, const float *dO,
+                                                          int B, float *G, const AdamArgs A) {
+    extern __shared__ __align__(16) float st[];
+    const int t = threadIdx.x, blk = blockIdx.x;
+    const bool is_w2 = blk < 16, is_w1 = blk >= 16 && blk < 22, is_w3 = blk == 24;
+    const float *s1 = is_w2 ? H1 : is_w3 ? H2 : blk == 23 ? dH2 : dH1;
+    const float *s2 = is_w2 ? dH2 + 4 * blk : is_w1 ? X : dO;
+    const int w2 = is_w1 ? F : is_w3 ? 1 : 0;  // floats a sample, contiguous (W2: four of H)
+    const bool by16 = ((reinterpret_cast<uintptr_t>(s1) | reinterpret_cast<uintptr_t>(s2)) & 15) == 0;
+    const int chunks = (B + GRAD_CHUNK - 1) / GRAD_CHUNK;
+    auto fetch = [&](int c) {
+        if (c < chunks) {
+            float *d1 = st + (c % GRAD_STAGES) * GRAD_STAGE_FLOATS, *d2 = d1 + GRAD_CHUNK * H;
+            const int b0 = c * GRAD_CHUNK, nb = min(GRAD_CHUNK, B - b0);
+            copy_run(d1, s1 + int64_t(b0) * H, nb * H, by16);
+            if (is_w2) {  // four of the columns
+                for (int e = t - ADD_THREADS; e < (by16 ? nb : 4 * nb); e += COPY_THREADS) {
+                    const int r = by16 ? e : e >> 2, o = by16 ? 0 : e & 3;
+                    copy_async(d2 + 4 * r + o, s2 + int64_t(b0 + r) * H + o, by16);
+                }
+            } else if (w2) {
+                copy_run(d2, s2 + int64_t(b0) * w2, nb * w2, by16);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const bool copies = t >= ADD_THREADS;
+    for (int c = 0; c < GRAD_STAGES - 1 && copies; c++) fetch(c);
+    const int col = t & 63, half = t >> 6;
+    float acc0 = 0.f, acc1 = 0.f;
+    for (int c = 0; c < chunks; c++) {
+        if (copies) asm volatile("cp.async.wait_group %0;" ::"n"(GRAD_STAGES - 2) : "memory");
+        __syncthreads();  // chunk c is there, and every thread is done with the chunk fetched over next
+        if (copies) {
+            fetch(c + GRAD_STAGES - 1);
+            continue;
+        }
+        const float *d1 = st + (c % GRAD_STAGES) * GRAD_STAGE_FLOATS, *d2 = d1 + GRAD_CHUNK * H;
+        const int nb = min(GRAD_CHUNK, B - c * GRAD_CHUNK);
+        if (is_w2) {
+            each_sample(nb, [&](int b) {
+                const float2 d = *reinterpret_cast<const float2 *>(d2 + b * 4 + 2 * half);
+                return make_float3(d1[b * H + col], d.x, d.y);
+            }, [&](float3 v) {
+                acc0 = fmaf(v.y, v.x, acc0);
+                acc1 = fmaf(v.z, v.x, acc1);
+            });
+        } else if (is_w1) {
+            const int i = 2 * (blk - 16) + half;
+            each_sample(nb, [&](int b) { return make_float2(d1[b * H + col], d2[b * F + i]); },
+                        [&](float2 v) { acc0 = fmaf(v.x, v.y, acc0); });
+        } else if (is_w3 && half == 0) {
+            each_sample(nb, [&](int b) { return make_float2(d2[b], d1[b * H + col]); },
+                        [&](float2 v) { acc0 = fmaf(v.x, v.y, acc0); });
+        } else if (is_w3 ? col == 0 : half == 0) {
+            each_sample(nb, [&](int b) { return is_w3 ? d2[b] : d1[b * H + col]; }, [&](float v) { acc0 += v; });
+        }
     }
-    const float m = b1 * M[p] + (1.f - b1) * g;
-    const float v = b2 * V[p] + (1.f - b2) * g * g;
-    M[p] = m;
-    V[p] = v;
-    P[p] -= lr * (m / c1) / (sqrtf(v / c2) + eps);
+    if (copies) return;
+    auto finish = [&](int p, float g) {
+        if (G) {
+            G[p] = g;
+            return;
+        }
+        const float m = A.b1 * A.M[p] + (1.f - A.b1) * g;
+        const float v = A.b2 * A.V[p] + (1.f - A.b2) * g * g;
+        A.M[p] = m;
+        A.V[p] = v;
+        A.P[p] -= A.lr * (m / A.c1) / (sqrtf(v / A.c2) + A.eps);
+    };
+    if (is_w2) {
+        const int j = 4 * blk + 2 * half;
+        finish(O_W2 + j * H + col, acc0);
+        finish(O_W2 + (j + 1) * H + col, acc1);
+    } else if (is_w1) {
+        finish(O_W1 + col * F + 2 * (blk - 16) + half, acc0);
+    } else if (is_w3) {
+        if (half == 0) finish(O_W3 + col, acc0);
+        else if (col == 0) finish(O_B3, acc0);
+    } else if (half == 0) {
+        finish((blk == 22 ? O_B1 : O_B2) + col, acc0);
+    }
 }
 
 __global__ void mlp_predict_kernel(const float *P, const float *X, int n, float *out) {
@@ -257,18 +319,22 @@ __global__ void mlp_pack_kernel(const float *P, const float *mean, const float *
     }
 }
 
-size_t scratch_floats(int B) { return size_t(B) * (4 * H + 1) + NPARAM + 4; }  // at least the partial sums
-
-// Launches the batch's gradients into rows of part (scratch), and returns how many rows.
-int grad_rows(const float *params, const float *features, const float *targets, int batch, float *part,
-              float *loss, cudaStream_t s) {
-    const int rows = std::min(MAX_ROWS, (batch + TS - 1) / TS);
-    cudaFuncSetAttribute(mlp_grad_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, GRAD_FLOATS * 4);
+// Launches the batch's passes and its gradients: into G, or one Adam step of A when G is NULL.
+void launch_step(const float *params, const float *features, const float *targets, int batch, float *scratch,
+                 float *G, const AdamArgs &A, float *loss, cudaStream_t s) {
+    float *H1 = scratch, *H2 = H1 + size_t(batch) * H, *dH1 = H2 + size_t(batch) * H;
+    float *dH2 = dH1 + size_t(batch) * H, *dO = dH2 + size_t(batch) * H;
+    const int threads = 256;
+    const int blocks = std::min(1184, (batch * 32 + threads - 1) / threads);
     cudaMemsetAsync(loss, 0, sizeof(float), s);
-    mlp_grad_tiles<<<rows, GRAD_THREADS, GRAD_FLOATS * sizeof(float), s>>>(params, features, targets, batch, part,
-                                                                            loss);
-    return rows;
+    mlp_fwd_bwd<<<blocks, threads, SMEM_FLOATS * sizeof(float), s>>>(params, features, targets,
+                                                                       batch, H1, H2, dH1, dH2, dO, loss);
+    constexpr int smem = GRAD_STAGES * GRAD_STAGE_FLOATS * 4;
+    cudaFuncSetAttribute(mlp_grads, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    mlp_grads<<<GRAD_BLOCKS, GRAD_THREADS, smem, s>>>(features, H1, H2, dH1, dH2, dO, batch, G, A);
 }
+
+size_t scratch_floats(int B) { return size_t(B) * (4 * H + 1) + NPARAM + 4; }
 
 }  // namespace hbm
 
@@ -293,11 +359,10 @@ int hnsw_b200_mlp_train_step(float *params, float *adam_m, float *adam_v, int64_
         step < 1)
         return hb::fail(HNSW_B200_EINVAL, "mlp_train_step: bad argument");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int rows = grad_rows(params, features, targets, batch, scratch, loss, s);
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - powf(b1, float(step)), c2 = 1.f - powf(b2, float(step));
-    mlp_finish<<<(NPARAM + FIN_PARAMS - 1) / FIN_PARAMS, 4 * FIN_PARAMS, 0, s>>>(
-        scratch, rows, nullptr, params, adam_m, adam_v, lr, b1, b2, 1e-8f, c1, c2);
+    launch_step(params, features, targets, batch, scratch, nullptr,
+                AdamArgs{params, adam_m, adam_v, lr, b1, b2, 1e-8f, c1, c2}, loss, s);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return hb::fail(HNSW_B200_ECUDA, std::string("mlp train: ") + cudaGetErrorString(e));
     return 0;
@@ -310,9 +375,7 @@ int hnsw_b200_mlp_gradients(const float *params, const float *features, const fl
     if (!params || !features || !targets || !scratch || !grads || !loss || batch < 1)
         return hb::fail(HNSW_B200_EINVAL, "mlp_gradients: bad argument");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int rows = grad_rows(params, features, targets, batch, scratch, loss, s);
-    mlp_finish<<<(NPARAM + FIN_PARAMS - 1) / FIN_PARAMS, 4 * FIN_PARAMS, 0, s>>>(
-        scratch, rows, grads, nullptr, nullptr, nullptr, 0.f, 0.f, 0.f, 0.f, 1.f, 1.f);
+    launch_step(params, features, targets, batch, scratch, grads, AdamArgs{}, loss, s);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return hb::fail(HNSW_B200_ECUDA, std::string("mlp grads: ") + cudaGetErrorString(e));
     return 0;
