@@ -23,6 +23,8 @@ METRIC_CODES = {"l2": L2, "ip": IP, "cosine": COSINE}
 DIST_F64 = 0
 DIST_EXACT_F32 = 1
 DIST_BYTES = 2
+# hnsw_b200_device_stats flags
+NOT_FINITE, ZERO_NORM, ROWS_NOT_FINITE, NOT_INTEGER = 1, 2, 4, 8
 
 
 class Graph(ctypes.Structure):
@@ -82,6 +84,16 @@ class SearchArgs(ctypes.Structure):
     ]
 
 
+class SearchExtra(ctypes.Structure):
+    """``hnsw_b200_search_extra_t``."""
+
+    _fields_ = [
+        ("totals", ctypes.c_void_p),
+        ("host_ids", ctypes.c_void_p),
+        ("host_dists", ctypes.c_void_p),
+    ]
+
+
 class ExactArgs(ctypes.Structure):
     _fields_ = [
         ("data", ctypes.c_void_p),
@@ -119,6 +131,8 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "hnsw_b200_open": (ctypes.c_int, [ctypes.POINTER(Graph), ctypes.POINTER(ctypes.c_void_p)]),
     "hnsw_b200_close": (None, [ctypes.c_void_p]),
     "hnsw_b200_search": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(SearchArgs), ctypes.c_void_p]),
+    "hnsw_b200_search_extra": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(SearchArgs),
+                                              ctypes.POINTER(SearchExtra), ctypes.c_void_p]),
     "hnsw_b200_exact_knn": (ctypes.c_int, [ctypes.POINTER(ExactArgs), ctypes.c_void_p]),
     "hnsw_b200_mlp_param_count": (ctypes.c_int64, []),
     "hnsw_b200_mlp_packed_bytes": (ctypes.c_int64, []),
@@ -150,6 +164,14 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "hnsw_b200_upload_queries": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64,
                                                 ctypes.c_int32, ctypes.POINTER(ValueStats),
                                                 ctypes.c_void_p, ctypes.c_void_p]),
+    "hnsw_b200_device_stats": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_int64,
+                                              ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p,
+                                              ctypes.POINTER(ctypes.c_uint32), ctypes.POINTER(ValueStats),
+                                              ctypes.c_void_p]),
+    "hnsw_b200_pack_mask": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p,
+                                           ctypes.c_void_p]),
+    "hnsw_b200_code_queries": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int64, ctypes.c_int32, ctypes.c_void_p,
+                                              ctypes.c_double, ctypes.c_void_p, ctypes.c_void_p]),
     "hnsw_b200_start_priority": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int64, ctypes.c_int32,
                                                 ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p,
                                                 ctypes.c_void_p, ctypes.c_float, ctypes.c_void_p,

@@ -200,6 +200,7 @@ struct SearchParams {
     int64_t *out_ids;
     double *out_dists;
     int64_t *out_ctr;
+    unsigned long long *totals;  // running sums of the counters over finished queries (2), or NULL
     int32_t *status;
     int32_t *n_failed;
     int32_t *queue;
@@ -2199,6 +2200,10 @@ __global__ void __launch_bounds__(WPB * 32, min_blocks<MODE, FILT, CFG>())
                 P.out_ctr[2 * int64_t(q)] = C.ndist;
                 P.out_ctr[2 * int64_t(q) + 1] = C.nhops;
             }
+            if (P.totals) {
+                atomicAdd(P.totals, static_cast<unsigned long long>(C.ndist));
+                atomicAdd(P.totals + 1, static_cast<unsigned long long>(C.nhops));
+            }
             if (P.cells) {  // the start order's per-cell cost table; cells outside it are skipped
                 const int c = P.cells[q];
                 if (c >= 0 && c < P.n_cells) {
@@ -2449,7 +2454,8 @@ namespace hb {
 // capture can record them); the scratch must already fit (a synchronous call with arguments of
 // the same size sized it), and overflowed queries stay unwritten with their count left on the
 // device for hnsw_b200_search_failed.
-int search_impl(Handle &h, const hnsw_b200_search_args_t *a, cudaStream_t s, bool async) {
+int search_impl(Handle &h, const hnsw_b200_search_args_t *a, cudaStream_t s, bool async,
+                const hnsw_b200_search_extra_t *ex = nullptr) {
     h.launches = 0;
     const hnsw_b200_graph_t &g = h.g;
     if (a->nq < 0 || a->nq > 0x7fffffff) return fail(HNSW_B200_EINVAL, "nq out of range");
@@ -2554,6 +2560,7 @@ int search_impl(Handle &h, const hnsw_b200_search_args_t *a, cudaStream_t s, boo
     P.out_ids = a->out_ids;
     P.out_dists = a->out_dists;
     P.out_ctr = a->out_counters;
+    P.totals = ex ? reinterpret_cast<unsigned long long *>(ex->totals) : nullptr;
     P.status = static_cast<int32_t *>(h.status.ptr);
     P.queue = ctr;
     P.n_failed = ctr + 1;
@@ -2642,6 +2649,13 @@ int search_impl(Handle &h, const hnsw_b200_search_args_t *a, cudaStream_t s, boo
         h.launches++;
         if (async) return 0;  // the overflow count stays on the device
         CUDA_TRY(cudaMemcpyAsync(h.host_pinned, ctr, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        // The results go to the host behind the same wait (a retry copies them again).
+        if (ex && ex->host_ids)
+            CUDA_TRY(cudaMemcpyAsync(ex->host_ids, a->out_ids, size_t(nq) * a->k * sizeof(int64_t),
+                                     cudaMemcpyDeviceToHost, s));
+        if (ex && ex->host_dists)
+            CUDA_TRY(cudaMemcpyAsync(ex->host_dists, a->out_dists, size_t(nq) * a->k * sizeof(double),
+                                     cudaMemcpyDeviceToHost, s));
         if (cudaStreamSynchronize(s) != cudaSuccess) {
             h.bits_dirty = true;
             return fail(HNSW_B200_ECUDA, std::string("search kernel failed: ") +
@@ -2678,6 +2692,14 @@ int hnsw_b200_search(void *handle, const hnsw_b200_search_args_t *a, void *strea
     Handle &h = *static_cast<Handle *>(handle);
     std::lock_guard<std::mutex> lock(h.mu);
     return search_impl(h, a, static_cast<cudaStream_t>(stream), false);
+}
+
+int hnsw_b200_search_extra(void *handle, const hnsw_b200_search_args_t *a, const hnsw_b200_search_extra_t *extra,
+                           void *stream) {
+    if (!handle || !a || !extra) return fail(HNSW_B200_EINVAL, "null argument");
+    Handle &h = *static_cast<Handle *>(handle);
+    std::lock_guard<std::mutex> lock(h.mu);
+    return search_impl(h, a, static_cast<cudaStream_t>(stream), false, extra);
 }
 
 int hnsw_b200_search_async(void *handle, const hnsw_b200_search_args_t *a, void *stream) {

@@ -47,6 +47,9 @@ NATIVE_FORMAT = "hnsw-engine-native"
 NATIVE_FORMAT_VERSION = 1
 NATIVE_HEADER = "header.json"
 SELECTIONS = ("simple", "heuristic")
+# Device query types whose NaN/inf check is that of their float32 or float64 values.
+_CHECKED_DTYPES = (torch.float32, torch.float64, torch.float16, torch.bfloat16, torch.uint8, torch.int8,
+                   torch.int16, torch.int32, torch.int64)
 
 
 @dataclass(frozen=True)
@@ -300,8 +303,8 @@ class HNSWIndex:
 
     def _device_queries(self, queries: torch.Tensor) -> _Uploaded:
         """Queries already on the GPU, with :meth:`_prepare`'s checks and messages (shape, real
-        dtype, width, NaN/inf, cosine zero rows, float32 overflow) and its values, read back as one
-        small copy that also carries the statistics picking the distance arithmetic."""
+        dtype, width, NaN/inf, cosine zero rows, float32 overflow) and its values: one launch and one
+        small read-back, which also carries the statistics picking the distance arithmetic."""
         if queries.ndim != 2:
             raise ValueError(f"vectors must be a 2-D array, got shape {tuple(queries.shape)}")
         if queries.dtype == torch.bool or queries.is_complex():
@@ -313,28 +316,26 @@ class HNSWIndex:
         with torch.cuda.device(queries.device):
             if queries.numel() == 0:
                 return _Uploaded(queries.to(torch.float32).contiguous(), _lib.DIST_F64)
-            raw_finite = torch.isfinite(queries).all()
-            zero_rows = torch.zeros((), dtype=torch.bool, device=queries.device)
+            if queries.dtype not in _CHECKED_DTYPES:
+                torch.isfinite(queries)  # raises where torch has no such check
+            norms = None
             if self._metric == "cosine":
                 q64 = queries.to(torch.float64)
                 norms = torch.linalg.norm(q64, dim=1, keepdim=True)
-                zero_rows = (norms == 0).any()
                 rows = (q64 / norms).to(torch.float32).contiguous()
+                raw = queries if queries.dtype == torch.float32 else q64
             else:
                 rows = queries.to(torch.float32).contiguous()
-            lo, hi = torch.aminmax(rows)
-            flags = torch.stack([raw_finite.double(), zero_rows.double(),
-                                 torch.isfinite(rows).all().double(),
-                                 (rows != torch.round(rows)).any().double(), lo.double(),
-                                 hi.double()]).cpu().tolist()
-        if not flags[0]:
+                raw = queries if queries.dtype == torch.float64 else rows
+            flags, st = g.device_stats(raw.contiguous(), None if raw is rows else rows, norms)
+        if flags & _lib.NOT_FINITE:
             raise ValueError("vectors contains NaN or infinite values")
-        if flags[1]:
+        if flags & _lib.ZERO_NORM:
             rows_host = torch.nonzero(norms[:, 0] == 0).flatten()[:5].cpu().tolist()
             raise ValueError(f"cosine distance is undefined for zero vectors (rows {rows_host})")
-        if not flags[2]:
+        if flags & _lib.ROWS_NOT_FINITE:
             raise ValueError("vectors overflow float32 (values beyond about 3.4e38)")
-        mode = g.choose_mode_device(rows, False, stats=(not flags[3], flags[4], flags[5]))
+        mode = g.choose_mode_device(rows, False, stats=(bool(st.integer), float(st.min), float(st.max)))
         return _Uploaded(rows, mode)
 
     def _check_search_args(self, k: int, ef: Any) -> tuple[int, Any]:
@@ -461,24 +462,22 @@ class HNSWIndex:
                 packed = stop.packed()
                 stop._packed_cache = packed
             stop_arg = (packed, stop.threshold, stop.slope, stop.slope_from)
-        ids, dists, ctr = g.search(prepared, k, ef, allowed=allowed, stop=stop_arg,
-                                   dist_mode=dist_mode)
-        self._accumulate(ctr)
-        if keep_device:
-            return ids, dists
-        # results into page-locked host memory, one synchronisation for both copies
-        ids_h = torch.empty(ids.shape, dtype=ids.dtype, pin_memory=True)
-        dists_h = torch.empty(dists.shape, dtype=dists.dtype, pin_memory=True)
-        ids_h.copy_(ids, non_blocking=True)
-        dists_h.copy_(dists, non_blocking=True)
-        torch.cuda.current_stream(g.device).synchronize()
-        return ids_h.numpy(), dists_h.numpy()
+        host_out = None
+        if not keep_device:  # results into page-locked host memory, behind the search's own wait
+            shape = (int(prepared.shape[0]), k)
+            host_out = (torch.empty(shape, dtype=torch.int64, pin_memory=True),
+                        torch.empty(shape, dtype=torch.float64, pin_memory=True))
+        ids, dists, _ = g.search(prepared, k, ef, allowed=allowed, stop=stop_arg, dist_mode=dist_mode,
+                                 counters=False, totals=self._totals(), host_out=host_out)
+        return (ids, dists) if host_out is None else (host_out[0].numpy(), host_out[1].numpy())
 
-    def _accumulate(self, ctr: torch.Tensor | None) -> None:
-        """Add a search's per-query counters to the running totals on the device (no sync)."""
-        if ctr is not None and ctr.numel():
-            s = ctr.sum(dim=0)
-            self._counters_dev = s if self._counters_dev is None else self._counters_dev + s
+    def _totals(self) -> torch.Tensor:
+        """The device-side counter sums that searches add to (read back by :meth:`_read_counters`)."""
+        if self._counters_dev is None:
+            dev = self.device_graph.device
+            self._counters_dev = torch.zeros(2, dtype=torch.int64, device=dev)
+            torch.cuda.current_stream(dev).synchronize()  # zero before a search on any stream adds to it
+        return self._counters_dev
 
     # ----------------------------------------------------------------------- inspection
     def stats(self) -> IndexStats:

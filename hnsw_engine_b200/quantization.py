@@ -166,18 +166,37 @@ class QuantizedIndex:
         if allowed is not None and not allowed.any():
             return np.full((nq, k_valid), -1, np.int64), np.full((nq, k_valid), np.inf)
         ef_fetch = np.maximum(np.asarray(ef_valid, dtype=np.int64), fetch)
-        code_q = self.quantizer.transform_queries(prepared, metric)
         g = self._index.device_graph
+        with torch.cuda.device(g.device):
+            # float32 rows go up; their code-space form (float64, twice the bytes) is made there
+            rows = torch.empty((nq, self._index.dim), dtype=torch.float32, device=g.device)
+            if nq:
+                g.upload_queries(prepared, rows)
+            code_q = self.transform_device(rows, metric)
+            mode = _lib.DIST_F64 if metric == "cosine" else g.choose_mode_device(code_q, True)
+            host = (torch.empty((nq, k_valid if r else fetch), dtype=torch.int64, pin_memory=True),
+                    torch.empty((nq, k_valid if r else fetch), dtype=torch.float64, pin_memory=True))
+        common = {"allowed": allowed, "use_codes": True, "dist_mode": mode, "counters": False,
+                  "totals": self._index._totals(), "host_out": host}
         if r == 0:
-            ids, dists, ctr = g.search(code_q, fetch, ef_fetch, allowed=allowed, use_codes=True)
-            self._index._accumulate(ctr)
-            return ids.cpu().numpy(), self.quantizer.to_distance(dists.cpu().numpy(), prepared, metric)
-        ids, dists, ctr = g.search(
-            code_q, k_valid, ef_fetch, allowed=allowed, use_codes=True, k_search=fetch,
-            rerank_queries=prepared,
-        )
-        self._index._accumulate(ctr)
-        return ids.cpu().numpy(), dists.cpu().numpy()
+            g.search(code_q, fetch, ef_fetch, **common)
+            return host[0].numpy(), self.quantizer.to_distance(host[1].numpy(), prepared, metric)
+        g.search(code_q, k_valid, ef_fetch, k_search=fetch, rerank_queries=rows, **common)
+        return host[0].numpy(), host[1].numpy()
+
+    def transform_device(self, prepared: torch.Tensor, metric: str) -> torch.Tensor:
+        """:meth:`ScalarQuantizer.transform_queries` of prepared float32 rows on the GPU: the same
+        float64 subtraction and division."""
+        out = torch.empty(prepared.shape, dtype=torch.float64, device=prepared.device)
+        offset = None
+        if metric == "l2":
+            offset = torch.from_numpy(np.ascontiguousarray(self.quantizer.offset, dtype=np.float64)).to(prepared.device)
+        stream = torch.cuda.current_stream(prepared.device).cuda_stream
+        _lib.check(_lib.load().hnsw_b200_code_queries(
+            prepared.data_ptr(), prepared.shape[0], prepared.shape[1],
+            None if offset is None else offset.data_ptr(), float(self.quantizer.step), out.data_ptr(),
+            ctypes.c_void_p(stream)))
+        return out
 
     def batch_search_device(self, code_queries: torch.Tensor, prepared: torch.Tensor, k: int,
                             ef: Any, rerank: int) -> tuple[torch.Tensor, torch.Tensor]:

@@ -215,6 +215,18 @@ void hnsw_b200_close(void *handle);
  * larger scratch; results are complete when it returns 0. */
 int hnsw_b200_search(void *handle, const hnsw_b200_search_args_t *args, void *stream);
 
+/* hnsw_b200_search with what a host caller would otherwise add launches and a second wait for: host_ids
+ * and host_dists (page-locked host memory of nq x k values, or NULL) receive the results behind the one
+ * wait, and totals (two int64 on the device, or NULL) gain the sums of the queries' distance
+ * computations and expansions. out_ids and out_dists are filled as by hnsw_b200_search. */
+typedef struct {
+    int64_t *totals;
+    int64_t *host_ids;
+    double *host_dists;
+} hnsw_b200_search_extra_t;
+int hnsw_b200_search_extra(void *handle, const hnsw_b200_search_args_t *args,
+                           const hnsw_b200_search_extra_t *extra, void *stream);
+
 /* The same search as hnsw_b200_search, issued with no host synchronisation, no allocation and
  * no host read, every launch on `stream`, so that it can be recorded in a CUDA graph and replayed
  * (the reference's search has no counterpart: it runs on the CPU). The handle's scratch must
@@ -317,6 +329,28 @@ typedef struct {
 } hnsw_b200_value_stats_t;
 int hnsw_b200_upload_queries(const float *src, float *dst, int64_t count, int32_t threads,
                              hnsw_b200_value_stats_t *out, float *staging, void *stream);
+
+/* The same of values on the GPU, in one launch: `count` float32 (float64: float64) values `raw` and, when
+ * rows is not NULL, the float32 rows prepared from them (else the values themselves), whose integrality,
+ * minimum and maximum are reported; norms: n_norms float64 row norms or NULL. *flags (host): the bits
+ * below. work: 24 bytes of device memory, 8-byte aligned. Synchronises the stream. */
+#define HNSW_B200_NOT_FINITE 1u       /* a raw value is NaN or +-inf */
+#define HNSW_B200_ZERO_NORM 2u        /* a norm is zero */
+#define HNSW_B200_ROWS_NOT_FINITE 4u  /* a prepared value is NaN or +-inf */
+#define HNSW_B200_NOT_INTEGER 8u      /* a prepared value is not an integer */
+int hnsw_b200_device_stats(const void *raw, int32_t float64, const float *rows, int64_t count,
+                           const double *norms, int64_t n_norms, void *work, uint32_t *flags,
+                           hnsw_b200_value_stats_t *out, void *stream);
+
+/* Filter bitmap of a mask on the GPU (one byte a node, by original id): bit i & 31 of word i >> 5 is
+ * mask[node_ids[i]] != 0 (node_ids NULL: mask[i]). bits: (n + 31) / 32 words. One launch. */
+int hnsw_b200_pack_mask(const uint8_t *mask, const int32_t *node_ids, int64_t n, uint32_t *bits,
+                        void *stream);
+
+/* Code-space queries (ScalarQuantizer.transform_queries, quantization.py:61-68) of prepared float32
+ * queries on the GPU: (double(x) - offset[j]) / step in float64, or double(x) when offset is NULL. */
+int hnsw_b200_code_queries(const float *queries, int64_t nq, int32_t dim, const double *offset,
+                           double step, double *out, void *stream);
 
 /* Start priorities for hnsw_b200_search (one launch): each query's cell -- its nearest of the
  * n_cells float32 pivot rows (squared L2 in float32, ties to the lower index) -- into cells, and
