@@ -34,7 +34,7 @@ import torch
 from numpy.typing import NDArray
 
 from . import _lib
-from .engine import DeviceGraph
+from .engine import DeviceGraph, to_device
 from .metrics import RELATIVE_TIE_TOLERANCE
 
 FEATURES = 12
@@ -173,7 +173,10 @@ class StopNetwork:
         """Adam on mean squared error over shuffled mini-batches (standardised features)."""
         self.mean = X.mean(axis=0).astype(np.float32)
         self.std = np.maximum(X.std(axis=0), 1e-6).astype(np.float32)
-        Xd = torch.from_numpy(self._norm(X)).to(self.device)
+        # standardised on the GPU, in _norm's float32 steps
+        Xd = to_device(np.asarray(X, dtype=np.float32), torch.float32, self.device)
+        Xd.sub_(torch.from_numpy(self.mean).to(self.device))
+        Xd.mul_(torch.from_numpy((1.0 / self.std).astype(np.float32)).to(self.device))
         yd = torch.from_numpy(np.ascontiguousarray(y, dtype=np.float32)).to(self.device)
         n = Xd.shape[0]
         scratch = torch.empty(int(self.lib.hnsw_b200_mlp_scratch_bytes(batch)) // 4 + 1,
@@ -186,9 +189,10 @@ class StopNetwork:
                 order = torch.randperm(n, generator=g).to(self.device)
                 ep_loss, nb = 0.0, 0
                 rate = lr * (0.5 ** ep)
+                used = order[: n // batch * batch]  # the epoch's samples in its order, gathered once
+                Xe, ye = Xd[used], yd[used]
                 for s in range(0, n - batch + 1, batch):
-                    idx = order[s : s + batch]
-                    xb, yb = Xd[idx].contiguous(), yd[idx].contiguous()
+                    xb, yb = Xe[s : s + batch], ye[s : s + batch]
                     self.step += 1
                     _lib.check(self.lib.hnsw_b200_mlp_train_step(
                         _ptr(self.params), _ptr(self.m), _ptr(self.v), self.step, rate, _ptr(xb),
