@@ -1,0 +1,45 @@
+"""Float64 code distances over the row widths and result capacities that choose their path."""
+
+from __future__ import annotations
+
+from functools import lru_cache
+
+import numpy as np
+import pytest
+from conftest import mix10k_arrays
+
+pytestmark = pytest.mark.gpu
+
+
+@lru_cache(maxsize=None)
+def _codes_case(dim: int, metric: str):
+    from hnsw_engine_b200 import HNSWIndex
+
+    arrays, ep, ml = mix10k_arrays()
+    n = arrays["vectors"].shape[0]
+    rng = np.random.default_rng(dim)
+    arrays = dict(arrays, vectors=rng.standard_normal((n, dim)).astype(np.float32))
+    codes = rng.integers(0, 256, (n, dim)).astype(np.uint8)
+    index = HNSWIndex.from_arrays(arrays, ep, ml, dim=dim, metric=metric, M=16)
+    index.device_graph.attach_codes(codes)
+    return index, arrays, ep, ml, codes
+
+
+# Widths: one word, part of a 128-byte piece, exactly one, one word more, several with a remainder; and rows
+# off 4-byte boundaries, which a lane reads by itself. ef: the largest tile, smaller ones and none.
+@pytest.mark.parametrize("dim,ef", [(4, 24), (36, 24), (128, 24), (132, 24), (260, 24), (6, 24), (33, 24),
+                                    (64, 400), (64, 900), (64, 2500)])
+@pytest.mark.parametrize("metric", ["l2", "ip", "cosine"])
+@pytest.mark.parametrize("filtered", [False, True])
+def test_code_rows_match_the_oracle(dim: int, ef: int, metric: str, filtered: bool) -> None:
+    from oracle import cpu
+
+    index, arrays, ep, ml, codes = _codes_case(dim, metric)
+    rng = np.random.default_rng(1)
+    queries = rng.standard_normal((12, dim)) * 100 + 120
+    mask = rng.random(codes.shape[0]) < 0.4 if filtered else None
+    ids, dists, ctr = index.device_graph.search(queries, 10, ef, allowed=mask, use_codes=True)
+    o_ids, o_d, o_c = cpu.search_batch(arrays, ep, ml, queries, 10, ef, metric, allowed=mask, codes=codes, threads=8)
+    np.testing.assert_array_equal(ids.cpu().numpy(), o_ids)
+    np.testing.assert_array_equal(dists.cpu().numpy(), o_d)
+    np.testing.assert_array_equal(ctr.cpu().numpy(), o_c)
