@@ -721,6 +721,7 @@ __device__ __forceinline__ void dists_bytes(const SearchParams &P, int32_t e, ui
     while (umask) {  // wide rows: NB / 2 rows at a time, every lane striding over the words
         constexpr int NW = NB / 2;
         int jj[NW];
+        uint32_t ej[NW];  // exchanged here: the loop over words has fewer rounds for some lanes
         uint32_t acc[NW];
 #pragma unroll
         for (int t = 0; t < NW; t++) {
@@ -729,6 +730,7 @@ __device__ __forceinline__ void dists_bytes(const SearchParams &P, int32_t e, ui
             if (umask) {
                 jj[t] = __ffs(umask) - 1;
                 umask &= umask - 1;
+                ej[t] = uint32_t(__shfl_sync(FULL, e, jj[t]));
             }
         }
         for (int w = lane; w < words; w += 32) {
@@ -736,8 +738,7 @@ __device__ __forceinline__ void dists_bytes(const SearchParams &P, int32_t e, ui
 #pragma unroll
             for (int t = 0; t < NW; t++) {
                 if (jj[t] < 0) continue;
-                const uint32_t ej = uint32_t(__shfl_sync(FULL, e, jj[t]));
-                const uint32_t x = __ldg(rows + size_t(ej) * words + w);
+                const uint32_t x = __ldg(rows + size_t(ej[t]) * words + w);
                 if (l2) {
                     const uint32_t d = __vabsdiffu4(x, q);
                     acc[t] = __dp4a(d, d, acc[t]);

@@ -1,4 +1,4 @@
-"""Float64 code distances over the row widths and result capacities that choose their path."""
+"""Code and byte rows over the widths and result capacities that choose their path."""
 
 from __future__ import annotations
 
@@ -43,3 +43,25 @@ def test_code_rows_match_the_oracle(dim: int, ef: int, metric: str, filtered: bo
     np.testing.assert_array_equal(ids.cpu().numpy(), o_ids)
     np.testing.assert_array_equal(dists.cpu().numpy(), o_d)
     np.testing.assert_array_equal(ctr.cpu().numpy(), o_c)
+
+
+# Byte rows of one word to several words a lane, those with words for some lanes only in the last round
+# (132, 200, 784) among them. Values to 99 keep every sum within a float32's whole numbers.
+@pytest.mark.parametrize("dim", [4, 96, 128, 132, 144, 200, 256, 260, 784])
+@pytest.mark.parametrize("metric", ["l2", "ip"])
+def test_byte_rows_match_the_oracle(dim: int, metric: str) -> None:
+    from hnsw_engine_b200 import HNSWIndex
+    from oracle import cpu
+
+    arrays, ep, ml = mix10k_arrays()
+    n = arrays["vectors"].shape[0]
+    rng = np.random.default_rng(dim)
+    arrays = dict(arrays, vectors=rng.integers(0, 100, (n, dim)).astype(np.float32))
+    index = HNSWIndex.from_arrays(arrays, ep, ml, dim=dim, metric=metric, M=16)
+    queries = rng.integers(0, 100, (40, dim)).astype(np.float32)
+    for mask in (None, rng.random(n) < 0.4):
+        ids, dists, ctr = index.device_graph.search(queries, 10, 48, allowed=mask, dist_mode=2)
+        o_ids, o_d, o_c = cpu.search_batch(arrays, ep, ml, queries, 10, 48, metric, allowed=mask, threads=8)
+        np.testing.assert_array_equal(ids.cpu().numpy(), o_ids)
+        np.testing.assert_array_equal(dists.cpu().numpy(), o_d)
+        np.testing.assert_array_equal(ctr.cpu().numpy(), o_c)
