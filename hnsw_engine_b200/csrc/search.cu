@@ -97,7 +97,7 @@ constexpr int WPB = 4;  // warps per block
 #define HB_CODE_WORDS 1
 #endif
 // Batched admission (unfiltered and filtered): rank a candidate in R (and in the filtered
-// candidates S) by a binary search whose step count depends on the array's length alone, so the
+// candidates S) by a search whose step count depends on the array's length alone, so the
 // lanes never diverge in it (uniform_prefix). Identical results; 1M mixture, 10K queries: ef = 192
 // 2.927 -> 2.907 ms, learned stop 3.04 -> 3.00 ms.
 #ifndef HB_UNIFORM_RANK
@@ -453,18 +453,67 @@ __device__ __forceinline__ void shift_down(T *Ad, int32_t *Ai, int pos, int m, i
 }
 
 // ---------------------------------------------------------------------------------------- visited
-// Length of the prefix of [0, m) on which pred holds (pred true on a prefix, false after), by a
-// binary search whose step count depends on m alone: the lanes of a warp never diverge in it.
+// Length of the prefix of [0, m) on which pred holds (pred true on a prefix, false after), by a search
+// whose step count depends on m alone: the lanes of a warp never diverge in it. Three places a step, read
+// together: what it costs is the steps' latency, half as many as a binary search's.
 template <class F>
 __device__ __forceinline__ int uniform_prefix(int m, F pred) {
-    int a = 0;  // the answer stays within [a, a + n]
-    for (int n = m; n > 1;) {
-        const int half = n >> 1;
-        a = pred(a + half - 1) ? a + half : a;
-        n -= half;
+    int a = 0, n = m;  // the answer stays within [a, a + n], a + n <= m
+    while (n > 3) {
+        const int h = n >> 2;
+        const int p1 = pred(a + h - 1), p2 = pred(a + 2 * h - 1), p3 = pred(a + 3 * h - 1);
+        a += h * (p1 + p2 + p3);
+        n -= 3 * h;
     }
-    if (m > 0 && pred(a)) a++;
-    return a;
+    const int p0 = n > 0 && pred(a), p1 = n > 1 && pred(a + 1), p2 = n > 2 && pred(a + 2);
+    return a + p0 + p1 + p2;
+}
+
+// Make room in a sorted array of n0 entries for n_add new ones, whose places in the result are f (one per
+// lane of `mine`, all different): every old entry moves up by the new ones below its new place. Two
+// windows of 32 places a step, highest first: every read of a step precedes its writes, and the writes
+// land above the next step's reads. Ap: an optional third array.
+template <typename T>
+__device__ __forceinline__ void make_room(T *Ad, int32_t *Ai, int32_t *Ap, int n0, int n_add, bool mine, int f,
+                                          int lane) {
+    const uint32_t below = (1u << lane) - 1u;
+    const int n = n0 + n_add;
+    int left = n_add;  // new entries below the windows still to do
+    for (int top = (n - 1) & ~63; top >= 0 && left > 0; top -= 64) {
+        const int w = top >> 5;
+        const uint32_t m1 = __reduce_or_sync(FULL, mine && (f >> 5) == w + 1 ? 1u << (f & 31) : 0u);
+        const uint32_t m0 = __reduce_or_sync(FULL, mine && (f >> 5) == w ? 1u << (f & 31) : 0u);
+        left -= __popc(m1);
+        const int t1 = top + 32 + lane, u1 = left + __popc(m1 & below);
+        left -= __popc(m0);
+        const int t0 = top + lane, u0 = left + __popc(m0 & below);
+        const bool a1 = t1 < n && u1 > 0 && t1 >= u1 && !((m1 >> lane) & 1u);
+        const bool a0 = t0 < n && u0 > 0 && t0 >= u0 && !((m0 >> lane) & 1u);
+        T d1 = T(0), d0 = T(0);
+        int32_t i1 = 0, i0 = 0, q1 = 0, q0 = 0;
+        if (a1) {
+            d1 = Ad[t1 - u1];
+            i1 = Ai[t1 - u1];
+            if (Ap) q1 = Ap[t1 - u1];
+        }
+        if (a0) {
+            d0 = Ad[t0 - u0];
+            i0 = Ai[t0 - u0];
+            if (Ap) q0 = Ap[t0 - u0];
+        }
+        __syncwarp();
+        if (a1) {
+            Ad[t1] = d1;
+            Ai[t1] = i1;
+            if (Ap) Ap[t1] = q1;
+        }
+        if (a0) {
+            Ad[t0] = d0;
+            Ai[t0] = i0;
+            if (Ap) Ap[t0] = q0;
+        }
+        __syncwarp();
+    }
 }
 
 __device__ __forceinline__ void vis_clear(int32_t *tab, int log2, int lane) {
@@ -1258,6 +1307,13 @@ __device__ __forceinline__ bool stop_checkpoint(const SearchParams &P, Cx &C, St
 // only if the worst distance did not drop, and gains the unexpanded evicted entries that tie the
 // final worst, pushed in descending (distance, id) order as the evictions would have pushed them.
 // churn (a stop feature) counts admissions that entered the first k at their insertion time.
+//
+// What bounds it is one warp's chain of shared reads, shuffles and branches, so: the rank by four-way
+// steps (uniform_prefix), four candidates' shuffles in flight, and room made by one mask of the new
+// places a window (make_room) instead of a count over the admitted per window. Kernel times on the 1M
+// mixture: 10K queries at ef = 192 3.05 -> 2.77 ms, 100 queries 637 -> 570 us, one query at ef = 64
+// 182 -> 170 us; 1M x 100 cosine in float64 4.67 -> 4.54 ms. (Eight candidates at once: 2.83 ms; four at
+// once in the filtered admission as well: 10.6 -> 10.8 ms, so that one keeps a candidate a step.)
 template <class Cx>
 __device__ __forceinline__ void admit_chunk(const SearchParams &P, Cx &C, int32_t e,
                                             typename Cx::dist_t dj, uint32_t um, int ef, int &r,
@@ -1296,14 +1352,25 @@ __device__ __forceinline__ void admit_chunk(const SearchParams &P, Cx &C, int32_
     // or below my distance, as lane masks.
     uint32_t ltm = 0u, plem = 0u, teq = 0u;  // teq: other candidates at my distance
     for (uint32_t m = cm; m;) {
-        const int i = __ffs(m) - 1;
-        m &= m - 1;
-        const D di = __shfl_sync(FULL, dj, i);
-        const uint32_t bit = 1u << i;
-        ltm |= di < dj ? bit : 0u;
-        teq |= (di == dj && i != lane) ? bit : 0u;
-        plem |= (i < lane && di <= dj) ? bit : 0u;
+        D di[4];
+        int ii[4];
+        uint32_t bit[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            bit[u] = m & (0u - m);
+            ii[u] = 31 - __clz(bit[u]);  // -1 past the last: no bit
+            m ^= bit[u];
+            di[u] = __shfl_sync(FULL, dj, ii[u] & 31);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            ltm |= di[u] < dj ? bit[u] : 0u;
+            teq |= di[u] == dj ? bit[u] : 0u;
+            plem |= di[u] <= dj ? bit[u] : 0u;
+        }
     }
+    teq &= ~(1u << lane);
+    plem &= (1u << lane) - 1u;
     if (__any_sync(FULL, teq != 0u)) {  // rare: equal distances order by original id
         const int32_t eo = inc ? orig_id(P, e) : -1;
         for (uint32_t m = cm; m;) {
@@ -1344,43 +1411,8 @@ __device__ __forceinline__ void admit_chunk(const SearchParams &P, Cx &C, int32_
     const int pos_r0 = lo + eq_lt;  // entries of R0 below (dj, e)
     const int fpos = pos_r0 + rank_a;
     churn += __popc(__ballot_sync(FULL, adm && pos_r0 + rank_prev < P.k));
-    const int pmin = __reduce_min_sync(FULL, adm ? pos_r0 : 0x7fffffff);
     const int fmin = __reduce_min_sync(FULL, adm ? fpos : 0x7fffffff);
-    // Move R0[p] (p >= pmin) up by the admitted entries that precede it, two chunks of 32 at a
-    // time, highest first: every entry of a step is read before any is written, and the writes
-    // land above every index the next step reads.
-    for (int top = r0 - 1; top >= pmin; top -= 64) {
-        const int p1 = top - lane, p2 = top - 32 - lane;
-        const bool a1 = p1 >= pmin, a2 = p2 >= pmin;
-        D d1 = D(0), d2 = D(0);
-        int32_t i1 = 0, i2 = 0;
-        if (a1) {
-            d1 = C.Rd[p1];
-            i1 = C.Ri[p1];
-        }
-        if (a2) {
-            d2 = C.Rd[p2];
-            i2 = C.Ri[p2];
-        }
-        int s1 = 0, s2 = 0;
-        for (uint32_t m = A; m;) {
-            const int i = __ffs(m) - 1;
-            m &= m - 1;
-            const int pr = __shfl_sync(FULL, pos_r0, i);
-            s1 += pr <= p1;
-            s2 += pr <= p2;
-        }
-        __syncwarp();
-        if (a1) {
-            C.Rd[p1 + s1] = d1;
-            C.Ri[p1 + s1] = i1;
-        }
-        if (a2) {
-            C.Rd[p2 + s2] = d2;
-            C.Ri[p2 + s2] = i2;
-        }
-        __syncwarp();
-    }
+    make_room(C.Rd, C.Ri, static_cast<int32_t *>(nullptr), r0, __popc(A), adm, fpos, lane);
     if (adm) {
         C.Rd[fpos] = dj;
         C.Ri[fpos] = e;
@@ -1766,46 +1798,8 @@ __device__ __forceinline__ void admit_chunk_filtered(const SearchParams &P, Cx &
     if (A) {
         const int pos_r0 = lo + eq_lt;  // R0 entries below (dj, eo)
         const int fpos = pos_r0 + __popc(ltm & A);
-        const int pmin = __reduce_min_sync(FULL, adm ? pos_r0 : 0x7fffffff);
         int32_t *rp = C.Rp != C.Ri ? C.Rp : nullptr;
-        // Move R0[p] (p >= pmin) up by the admissions before it, two chunks of 32 a step, highest
-        // first (every read of a step precedes its writes; writes land above the next step's reads).
-        for (int top = r0 - 1; top >= pmin; top -= 64) {
-            const int p1 = top - lane, p2 = top - 32 - lane;
-            const bool a1 = p1 >= pmin, a2 = p2 >= pmin;
-            D d1 = D(0), d2 = D(0);
-            int32_t i1 = 0, i2 = 0, q1 = 0, q2 = 0;
-            if (a1) {
-                d1 = C.Rd[p1];
-                i1 = C.Ri[p1];
-                if (rp) q1 = rp[p1];
-            }
-            if (a2) {
-                d2 = C.Rd[p2];
-                i2 = C.Ri[p2];
-                if (rp) q2 = rp[p2];
-            }
-            int s1 = 0, s2 = 0;
-            for (uint32_t m = A; m;) {
-                const int i = __ffs(m) - 1;
-                m &= m - 1;
-                const int pr = __shfl_sync(FULL, pos_r0, i);
-                s1 += pr <= p1;
-                s2 += pr <= p2;
-            }
-            __syncwarp();
-            if (a1) {
-                C.Rd[p1 + s1] = d1;
-                C.Ri[p1 + s1] = i1;
-                if (rp) rp[p1 + s1] = q1;
-            }
-            if (a2) {
-                C.Rd[p2 + s2] = d2;
-                C.Ri[p2 + s2] = i2;
-                if (rp) rp[p2 + s2] = q2;
-            }
-            __syncwarp();
-        }
+        make_room(C.Rd, C.Ri, rp, r0, __popc(A), adm, fpos, lane);
         if (adm) {
             C.Rd[fpos] = dj;
             C.Ri[fpos] = eo;
@@ -1931,46 +1925,9 @@ __device__ __forceinline__ void admit_chunk_filtered(const SearchParams &P, Cx &
     const int s1 = s0 - x0;
     if (RM) {
         const bool mine = (RM >> lane) & 1u;
-        const int ins = s_above - x0;
-        const int pmin = __reduce_min_sync(FULL, mine ? ins : 0x7fffffff);
-        for (int top = s1 - 1; top >= pmin; top -= 64) {
-            const int p1 = top - lane, p2 = top - 32 - lane;
-            const bool a1 = p1 >= pmin, a2 = p2 >= pmin;
-            D d1 = D(0), d2 = D(0);
-            int32_t i1 = 0, i2 = 0, q1 = 0, q2 = 0;
-            if (a1) {
-                d1 = C.Sd[p1];
-                i1 = C.Si[p1];
-                if (sp) q1 = sp[p1];
-            }
-            if (a2) {
-                d2 = C.Sd[p2];
-                i2 = C.Si[p2];
-                if (sp) q2 = sp[p2];
-            }
-            int u1 = 0, u2 = 0;
-            for (uint32_t m = RM; m;) {
-                const int i = __ffs(m) - 1;
-                m &= m - 1;
-                const int pi = __shfl_sync(FULL, ins, i);
-                u1 += pi <= p1;
-                u2 += pi <= p2;
-            }
-            __syncwarp();
-            if (a1) {
-                C.Sd[p1 + u1] = d1;
-                C.Si[p1 + u1] = i1;
-                if (sp) sp[p1 + u1] = q1;
-            }
-            if (a2) {
-                C.Sd[p2 + u2] = d2;
-                C.Si[p2 + u2] = i2;
-                if (sp) sp[p2 + u2] = q2;
-            }
-            __syncwarp();
-        }
+        const int f = rank_new - excess;
+        make_room(C.Sd, C.Si, sp, s1, __popc(RM), mine, f, lane);
         if (mine) {
-            const int f = rank_new - excess;
             C.Sd[f] = dj;
             C.Si[f] = eo;
             if (sp) sp[f] = e;
