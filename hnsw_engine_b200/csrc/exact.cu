@@ -316,6 +316,9 @@ struct EpiThread {
                     cnt++;
                 }
             }
+            // The lanes part above, and the TMEM instructions that follow (the next group's load, the
+            // caller's wait) are .aligned: the whole warp has to execute them together.
+            __syncwarp();
         }
     }
 };
