@@ -1277,8 +1277,15 @@ size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 // Candidate lists take at most CAND_BYTES of scratch: (query, segment) pairs x cap x 8 bytes.
 constexpr int64_t CAND_BYTES = int64_t(4) << 30;
 constexpr int64_t MAX_CHUNK = 16384;  // queries of a batch filtered together
-// Lists are sized for EXPECT_FACTOR times the candidates that pass two is expected to keep.
-constexpr int64_t EXPECT_FACTOR = 2;
+// A segment of pass two is sized for SEGMENT_FACTOR times its even share of the candidates expected, for
+// thresholds looser than expected and uneven shares, and for SEGMENT_SLACK entries more: the columns it has
+// in two tiles, for rows stored by cluster or by time, whose near rows lie in one or two tiles of one
+// segment. With half a tile's columns of slack (32) such rows overflowed and the call ran twice: 10K
+// queries x 1M x 128 bytes in 10,000 runs of similar rows, k = 100, 8.36 -> 4.20 ms; 2,000 x 200K x 64 floats
+// in 10,000 runs, k = 10, 936 -> 480 us; rows in no order take the same time with either (3.21 ms,
+// 430 us). Longer runs still overflow (1,000 rows each: 12.6 ms).
+constexpr int64_t SEGMENT_FACTOR = 6;
+constexpr int64_t SEGMENT_SLACK = 4 * CW;
 // Byte rows use the integer filter (1) or the BF16 one (0).
 #ifndef HB_EXACT_I8
 #define HB_EXACT_I8 1
@@ -1382,8 +1389,9 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
     // Pass one keeps the minimum of every block of two tiles' chunks of an epilogue thread (every row when
     // the sample has fewer than k blocks); pass two keeps the rows within tau + margin. Each epilogue
     // thread appends to its own segment of the query's list: in pass one at most one entry per block
-    // or its 2 CW columns of a tile; pass two's segments are sized for three times their expected share
-    // (an overflow re-runs the call with longer segments).
+    // or its 2 CW columns of a tile; pass two's segments get SEGMENT_FACTOR times their even share of the
+    // expected candidates and SEGMENT_SLACK more, and never more than the columns that they cover (an
+    // overflow re-runs the call with longer segments).
     const int tiles = int((n + BN - 1) / BN);
     const int64_t sample_rows = std::min<int64_t>(
         n, std::max<int64_t>(int64_t(64) * k, int64_t(std::sqrt(SAMPLE_BALANCE * double(k) * double(n)))));
@@ -1391,18 +1399,18 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
     const int sample = (tiles + stride - 1) / stride;  // tiles 0, stride, 2 stride, ... of pass one
     const bool block_min = int64_t(sample) / 2 * EPI_PER_QUARTER >= k;
     const int rank = sample_rank(k, sample, tiles);
-    const int64_t expect2 = EXPECT_FACTOR * (int64_t(rank) * tiles / sample) + int64_t(k);
+    const int64_t expect2 = int64_t(rank) * tiles / sample + int64_t(k) / 2;  // candidates of a query
     int64_t QB = std::min<int64_t>(nq_all, MAX_CHUNK);  // queries per chunk
     int64_t cap = 0, slots = 0;                           // entries per segment; (query, segment) pairs
     for (;;) {
-        cap = std::min<int64_t>(cap_min, n);
-        slots = 0;
+        cap = slots = 0;
         const int64_t last = nq_all % QB ? nq_all % QB : QB;
         for (int64_t nqc : {QB, last}) {
             const Geo g1 = geo(nqc, sample), g2 = geo(nqc, tiles);
             const int64_t nseg2 = int64_t(g2.splits) * EPI_PER_QUARTER;
+            const int64_t share = (SEGMENT_FACTOR * expect2 + nseg2 - 1) / nseg2 + SEGMENT_SLACK;
             cap = std::max<int64_t>(cap, block_min ? (g1.tps + 1) / 2 : int64_t(2 * CW) * g1.tps);
-            cap = std::max<int64_t>(cap, (3 * expect2 + nseg2 - 1) / nseg2 + 32);
+            cap = std::max<int64_t>(cap, std::min<int64_t>(std::max(cap_min, share), int64_t(2 * CW) * g2.tps));
             slots = std::max<int64_t>(slots, nqc * std::max(g1.splits, g2.splits) * EPI_PER_QUARTER);
         }
         if (slots * cap * 8 <= CAND_BYTES || QB <= BM) break;
@@ -1628,7 +1636,7 @@ extern "C" int hnsw_b200_exact_knn(const hnsw_b200_exact_args_t *a, void *stream
         return fail(HNSW_B200_EINVAL, "unsupported dtype");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     // A candidate overflow re-runs the batch with lists long enough for the largest count seen
-    // (plus a quarter); a list of n entries can never overflow, so this ends.
+    // (plus a quarter); a segment as long as the columns it covers cannot overflow, so this ends.
     int64_t cap_min = 0;
     for (int attempt = 0; attempt < 4; attempt++) {
         int64_t need = 0;
