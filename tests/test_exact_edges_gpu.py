@@ -61,3 +61,57 @@ def test_rows_stored_by_cluster_fit_the_first_lists(n: int, dim: int, nq: int, r
     o_ids, o_d = exact.exact_search(data, queries[:64], k, "l2")
     np.testing.assert_array_equal(ids[:64].cpu().numpy(), o_ids)
     np.testing.assert_allclose(dists[:64].cpu().numpy(), o_d, rtol=0 if as_bytes else dim * 2.0**-52)
+
+
+def _cosine_nan_last(data: np.ndarray, queries: np.ndarray, k: int) -> tuple[np.ndarray, np.ndarray]:
+    """Exact cosine order by (distance, id) with undefined distances (zero rows or queries) last."""
+    x, q = data.astype(np.float64), queries.astype(np.float64)
+    with np.errstate(invalid="ignore", divide="ignore"):
+        x, q = x / np.linalg.norm(x, axis=1)[:, None], q / np.linalg.norm(q, axis=1)[:, None]
+    d = 1.0 - q @ x.T
+    ids = np.argsort(d, axis=1, kind="stable")[:, :k]  # NumPy sorts NaN last
+    return ids, np.take_along_axis(d, ids, axis=1)
+
+
+@pytest.mark.parametrize("dim", [24, 300])        # a lane's sums, the warp's sums
+@pytest.mark.parametrize("n,k", [
+    (1, 1), (33, 33), (300, 300),  # every row a result
+    (300, 40),                     # some
+    (5_000, 3_000),                # too many to gather: inserted
+])
+def test_zero_rows_and_queries_under_cosine_come_last(dim: int, n: int, k: int) -> None:
+    """Rows on the GPU are taken as they are: a zero row's distance is NaN, and it comes after every
+    other result, by id among its like; a zero query's results are the first rows."""
+    import torch
+
+    from hnsw_engine_b200.exact_knn import exact_search
+
+    rng = np.random.default_rng(n + dim)
+    data = rng.standard_normal((n, dim)).astype(np.float32)
+    # in the second half of the directions every distance of the first queries is above 1, the filter
+    # value of a zero row, so zero rows are within the threshold
+    data[:, 0] = -np.abs(data[:, 0]) - 4.0
+    data[rng.permutation(n)[: max(1, n // 50)]] = 0.0
+    queries = rng.standard_normal((5, dim)).astype(np.float32)
+    queries[:, 0] = 8.0
+    queries[3] = 0.0
+    ids, dists = exact_search(torch.from_numpy(data).cuda(), torch.from_numpy(queries).cuda(), k, "cosine")
+    ids, dists = ids.cpu().numpy(), dists.cpu().numpy()
+    if k == n:
+        w_ids, w_d = _cosine_nan_last(data, queries, k)
+        np.testing.assert_allclose(dists, w_d, rtol=0, atol=dim * 2.0**-52)
+        np.testing.assert_array_equal(ids, w_ids)
+        return
+    norms = np.linalg.norm(data, axis=1)
+    for i in range(len(queries)):
+        assert np.unique(ids[i]).size == k and (ids[i] >= 0).all() and (ids[i] < n).all()
+        nan = np.isnan(dists[i])
+        m = int((~nan).sum())
+        assert not nan[:m].any() and (np.diff(dists[i, :m]) >= 0).all()
+        assert (np.diff(ids[i, m:]) > 0).all()
+        if i == 3:
+            assert m == 0
+            continue
+        assert (norms[ids[i, m:]] == 0).all() and (norms[ids[i, :m]] > 0).all()
+        _, w_d = _cosine_nan_last(data[norms > 0], queries[i : i + 1], max(m, 1))
+        np.testing.assert_allclose(dists[i, :m], w_d[0, :m], rtol=0, atol=dim * 2.0**-52)
