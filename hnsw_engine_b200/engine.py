@@ -15,6 +15,7 @@ over the dimensions, which is the reference's own arithmetic (``_distance``, num
 from __future__ import annotations
 
 import ctypes
+import threading
 import warnings
 from typing import Any
 
@@ -206,6 +207,7 @@ class DeviceGraph:
         # page-locked staging of uploaded query batches, and the end of the last DMA from it
         self._stage: torch.Tensor | None = None
         self._stage_done = torch.cuda.Event()
+        self._stage_lock = threading.Lock()
         self._internal: dict[str, Any] = {}
         # Runtime autotuner (see search): kernel configuration per tune_key, with the timings that
         # chose it.
@@ -442,18 +444,23 @@ class DeviceGraph:
             raise ValueError("dst must be a contiguous float32 device tensor of src's size")
         with torch.cuda.device(self.device):
             stream = torch.cuda.current_stream(self.device)
-            stage = None
-            if staged:
+
+            def upload(stage: torch.Tensor | None) -> None:
+                _lib.check(self.lib.hnsw_b200_upload_queries(
+                    src.ctypes.data, _dev_ptr(dst), src.size, int(threads), ctypes.byref(st),
+                    _dev_ptr(stage), ctypes.c_void_p(stream.cuda_stream)))
+
+            if not staged:
+                upload(None)
+                return st
+            # One buffer for every caller: from the first row staged in it until the event that the
+            # next caller waits for, it is this call's alone (the library call lets other threads run).
+            with self._stage_lock:
+                self._stage_done.synchronize()  # the previous DMA from it has finished
                 if self._stage is None or self._stage.numel() < src.size:
                     self._stage = torch.empty(max(src.size, 1 << 20), dtype=torch.float32,
                                               pin_memory=True)
-                else:
-                    self._stage_done.synchronize()  # the previous DMA from it has finished
-                stage = self._stage
-            _lib.check(self.lib.hnsw_b200_upload_queries(
-                src.ctypes.data, _dev_ptr(dst), src.size, int(threads), ctypes.byref(st),
-                _dev_ptr(stage), ctypes.c_void_p(stream.cuda_stream)))
-            if stage is not None:
+                upload(self._stage)
                 self._stage_done.record(stream)
         return st
 

@@ -1,0 +1,75 @@
+"""One graph used by several threads: the buffers that its calls share, with the library replaced by
+functions that do its copies on the host, slowly, while other threads run."""
+
+from __future__ import annotations
+
+import ctypes
+import threading
+import time
+from contextlib import nullcontext
+from types import SimpleNamespace
+
+import numpy as np
+import pytest
+
+
+@pytest.fixture
+def host_graph(monkeypatch: pytest.MonkeyPatch):
+    """A DeviceGraph without a GPU: its device is the host, and nothing of its graph is set."""
+    import torch
+
+    from hnsw_engine_b200.engine import DeviceGraph
+
+    monkeypatch.setattr(torch.cuda, "device", lambda dev: nullcontext())
+    stream = SimpleNamespace(cuda_stream=0, synchronize=lambda: None)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: stream)
+    empty = torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *a, pin_memory=False, **kw: empty(*a, **kw))
+    g = DeviceGraph.__new__(DeviceGraph)
+    g.device = torch.device("cpu")
+    g.dim = 8
+    g._stage = None
+    g._stage_done = SimpleNamespace(synchronize=lambda: None, record=lambda stream: None)
+    g._stage_lock = threading.Lock()
+    return g
+
+
+def _together(work, count: int) -> None:
+    """work(0) .. work(count - 1) on a thread each; the first error is raised here."""
+    errors: list[BaseException] = []
+    gate = threading.Barrier(count)
+
+    def body(i: int) -> None:
+        try:
+            gate.wait()
+            work(i)
+        except BaseException as e:  # noqa: BLE001 - reported below
+            errors.append(e)
+
+    threads = [threading.Thread(target=body, args=(i,)) for i in range(count)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    if errors:
+        raise errors[0]
+
+
+def test_threads_upload_their_own_rows(host_graph) -> None:
+    """Every upload of a graph goes through one staging buffer."""
+    import torch
+
+    def upload(src, dst, count, threads, stats, stage, stream):
+        ctypes.memmove(stage, src, count * 4)
+        time.sleep(0.05)  # another thread runs here, as it does while the library stages rows
+        ctypes.memmove(dst, stage, count * 4)
+        return 0
+
+    g = host_graph
+    g.lib = SimpleNamespace(hnsw_b200_upload_queries=upload)
+    rows = [np.full((64 + i, 8), float(i), dtype=np.float32) for i in range(6)]
+    out = [torch.full(r.shape, -1.0) for r in rows]
+    g.upload_queries(rows[0], out[0])  # the buffer is there before the threads are
+    _together(lambda i: g.upload_queries(rows[i], out[i]), len(rows))
+    for r, o in zip(rows, out):
+        np.testing.assert_array_equal(o.numpy(), r)
