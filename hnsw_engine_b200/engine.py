@@ -208,6 +208,7 @@ class DeviceGraph:
         self._stage: torch.Tensor | None = None
         self._stage_done = torch.cuda.Event()
         self._stage_lock = threading.Lock()
+        self.counters_lock = threading.Lock()  # of the index's device-side counter sums
         self._internal: dict[str, Any] = {}
         # Runtime autotuner (see search): kernel configuration per tune_key, with the timings that
         # chose it.

@@ -158,7 +158,8 @@ class HNSWIndex:
         self._arrays: dict[str, NDArray[Any]] | None = None
         self._size = 0
         self._counters = np.zeros(2, dtype=np.int64)  # distance computations, hops
-        self._counters_dev: torch.Tensor | None = None  # device-side share not yet read back
+        self._counters_dev: torch.Tensor | None = None  # device-side sums of the index's lifetime
+        self._counters_seen = np.zeros(2, dtype=np.int64)  # their share that _counters holds already
         self._meta_extra: dict[str, Any] = {}
 
     # ----------------------------------------------------------------------- opening
@@ -248,10 +249,13 @@ class HNSWIndex:
         return int(self._read_counters()[1])
 
     def _read_counters(self) -> NDArray[np.int64]:
-        """Fold the searches' device-side counter sums into the host totals (one small copy)."""
+        """Fold what the searches' device-side sums gained into the host totals (one small copy). The
+        sums stay: a search in flight in another thread adds to them, and the next reading has it."""
         if self._counters_dev is not None:
-            self._counters += self._counters_dev.cpu().numpy()
-            self._counters_dev = None
+            with self.device_graph.counters_lock:
+                now = self._counters_dev.cpu().numpy().copy()
+                self._counters += now - self._counters_seen
+                self._counters_seen = now
         return self._counters
 
     def native_arrays(self) -> dict[str, NDArray[Any]]:
@@ -473,11 +477,14 @@ class HNSWIndex:
 
     def _totals(self) -> torch.Tensor:
         """The device-side counter sums that searches add to (read back by :meth:`_read_counters`)."""
-        if self._counters_dev is None:
-            dev = self.device_graph.device
-            self._counters_dev = torch.zeros(2, dtype=torch.int64, device=dev)
-            torch.cuda.current_stream(dev).synchronize()  # zero before a search on any stream adds to it
-        return self._counters_dev
+        g = self.device_graph
+        with g.counters_lock:
+            if self._counters_dev is None:
+                dev = g.device
+                sums = torch.zeros(2, dtype=torch.int64, device=dev)
+                torch.cuda.current_stream(dev).synchronize()  # zero before a search on any stream adds
+                self._counters_dev = sums
+            return self._counters_dev
 
     # ----------------------------------------------------------------------- inspection
     def stats(self) -> IndexStats:
@@ -513,8 +520,8 @@ class HNSWIndex:
         )
 
     def reset_counters(self) -> None:
+        self._read_counters()
         self._counters[:] = 0
-        self._counters_dev = None
 
     def _params(self) -> dict[str, Any]:
         return {

@@ -31,6 +31,7 @@ def host_graph(monkeypatch: pytest.MonkeyPatch):
     g._stage = None
     g._stage_done = SimpleNamespace(synchronize=lambda: None, record=lambda stream: None)
     g._stage_lock = threading.Lock()
+    g.counters_lock = threading.Lock()
     return g
 
 
@@ -73,3 +74,25 @@ def test_threads_upload_their_own_rows(host_graph) -> None:
     _together(lambda i: g.upload_queries(rows[i], out[i]), len(rows))
     for r, o in zip(rows, out):
         np.testing.assert_array_equal(o.numpy(), r)
+
+
+def test_counters_read_during_a_search_keep_its_share(host_graph) -> None:
+    """A search in flight adds to the sums that it was given; reading or resetting the counters meanwhile
+    takes what is there and leaves the rest to the next reading."""
+    from hnsw_engine_b200 import HNSWIndex
+
+    index = HNSWIndex(8, "l2")
+    index._graph = host_graph
+    sums = index._totals()
+    sums += 5
+    assert (index.distance_computations, index.hops) == (5, 5)
+    sums += 7  # the search that began before the reading ends after it
+    assert (index.distance_computations, index.hops) == (12, 12)
+    assert (index.distance_computations, index.hops) == (12, 12)
+    index.reset_counters()
+    assert (index.distance_computations, index.hops) == (0, 0)
+    sums += 3
+    assert (index.distance_computations, index.hops) == (3, 3)
+    got: list[int] = []
+    _together(lambda i: got.append(index._totals().data_ptr()), 8)
+    assert set(got) == {sums.data_ptr()}
