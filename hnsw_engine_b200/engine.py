@@ -208,6 +208,8 @@ class DeviceGraph:
         self._stage: torch.Tensor | None = None
         self._stage_done = torch.cuda.Event()
         self._stage_lock = threading.Lock()
+        self._one: dict[str, Any] | None = None  # search_one's buffers
+        self._one_lock = threading.Lock()
         self.counters_lock = threading.Lock()  # of the index's device-side counter sums
         self._internal: dict[str, Any] = {}
         # Runtime autotuner (see search): kernel configuration per tune_key, with the timings that
@@ -532,36 +534,42 @@ class DeviceGraph:
         the copies' launches and gaps would cost more than the bus), the arithmetic is chosen on the
         host from the query's own values, and one library call waits once. Returns host arrays
         (ids (k,), distances (k,), counters (2,))."""
-        dev = self.device
         key = int(k)
-        buf = getattr(self, "_one", None)
-        if buf is None or buf["k"] != key:
-            with torch.cuda.device(dev):
-                buf = {
-                    "k": key,
-                    "q": torch.empty((1, self.dim), dtype=torch.float32, pin_memory=True),
-                    "ef": torch.empty(1, dtype=torch.int32, pin_memory=True),
-                    "ids": torch.empty((1, key), dtype=torch.int64, pin_memory=True),
-                    "dists": torch.empty((1, key), dtype=torch.float64, pin_memory=True),
-                    "ctr": torch.empty((1, 2), dtype=torch.int64, pin_memory=True),
-                }
-            buf["views"] = {name: buf[name].numpy() for name in ("q", "ef", "ids", "dists", "ctr")}
-            buf["args"] = _lib.SearchArgs(
-                queries=buf["q"].data_ptr(), queries_f64=0, use_codes=0, nq=1, k=key, k_search=key,
-                ef=buf["ef"].data_ptr(), allowed=None, allowed_fraction=1.0, rerank_queries=None,
-                out_ids=buf["ids"].data_ptr(), out_dists=buf["dists"].data_ptr(),
-                out_counters=buf["ctr"].data_ptr(),
-            )
-            self._one = buf
         q = np.asarray(query, dtype=np.float32).reshape(1, self.dim)
-        view, args = buf["views"], buf["args"]
-        view["q"][:] = q
-        view["ef"][0] = args.ef_max = max(int(ef), key)
-        args.dist_mode = int(self.choose_mode(q, False))
-        with torch.cuda.device(dev):
-            stream = torch.cuda.current_stream(dev).cuda_stream
-            _lib.check(self.lib.hnsw_b200_search(self._handle, ctypes.byref(args), ctypes.c_void_p(stream)))
-        return view["ids"][0].copy(), view["dists"][0].copy(), view["ctr"][0].copy()
+        mode = int(self.choose_mode(q, False))
+        # One set of buffers: it is this call's alone until its results are copied out (the library call
+        # lets other threads run, and searches of one graph follow each other there anyway).
+        with self._one_lock:
+            buf = self._one
+            if buf is None or buf["k"] != key:
+                buf = self._one = self._one_buffers(key)
+            view, args = buf["views"], buf["args"]
+            view["q"][:] = q
+            view["ef"][0] = args.ef_max = max(int(ef), key)
+            args.dist_mode = mode
+            with torch.cuda.device(self.device):
+                stream = torch.cuda.current_stream(self.device).cuda_stream
+                _lib.check(self.lib.hnsw_b200_search(self._handle, ctypes.byref(args), ctypes.c_void_p(stream)))
+            return view["ids"][0].copy(), view["dists"][0].copy(), view["ctr"][0].copy()
+
+    def _one_buffers(self, k: int) -> dict[str, Any]:
+        """:meth:`search_one`'s page-locked query, efSearch and results for k results, and its arguments."""
+        with torch.cuda.device(self.device):
+            buf: dict[str, Any] = {
+                "q": torch.empty((1, self.dim), dtype=torch.float32, pin_memory=True),
+                "ef": torch.empty(1, dtype=torch.int32, pin_memory=True),
+                "ids": torch.empty((1, k), dtype=torch.int64, pin_memory=True),
+                "dists": torch.empty((1, k), dtype=torch.float64, pin_memory=True),
+                "ctr": torch.empty((1, 2), dtype=torch.int64, pin_memory=True),
+            }
+        args = _lib.SearchArgs(
+            queries=buf["q"].data_ptr(), queries_f64=0, use_codes=0, nq=1, k=k, k_search=k,
+            ef=buf["ef"].data_ptr(), allowed=None, allowed_fraction=1.0, rerank_queries=None,
+            out_ids=buf["ids"].data_ptr(), out_dists=buf["dists"].data_ptr(),
+            out_counters=buf["ctr"].data_ptr(),
+        )
+        views = {name: t.numpy() for name, t in buf.items()}
+        return {**buf, "k": k, "views": views, "args": args}
 
     # ------------------------------------------------------------------------------ search
     def search(

@@ -32,6 +32,10 @@ def host_graph(monkeypatch: pytest.MonkeyPatch):
     g._stage_done = SimpleNamespace(synchronize=lambda: None, record=lambda stream: None)
     g._stage_lock = threading.Lock()
     g.counters_lock = threading.Lock()
+    g._one = None
+    g._one_lock = threading.Lock()
+    g._handle = ctypes.c_void_p()
+    g.choose_mode = lambda q, codes: 0
     return g
 
 
@@ -96,3 +100,35 @@ def test_counters_read_during_a_search_keep_its_share(host_graph) -> None:
     got: list[int] = []
     _together(lambda i: got.append(index._totals().data_ptr()), 8)
     assert set(got) == {sums.data_ptr()}
+
+
+@pytest.mark.parametrize("ks", [[4] * 6, [3, 4, 5, 3, 4, 5]])
+def test_threads_get_their_own_single_results(host_graph, ks: list[int]) -> None:
+    """Single searches of a graph share the page-locked query and results."""
+    g = host_graph
+
+    def values(address, ctype, count):
+        return np.ctypeslib.as_array(ctypes.cast(address, ctypes.POINTER(ctype)), (count,))
+
+    def search(handle, args_ref, stream):
+        args = args_ref._obj
+        q, k = values(args.queries, ctypes.c_float, g.dim)[0], args.k
+        ef = values(args.ef, ctypes.c_int32, 1)[0]
+        values(args.out_ids, ctypes.c_int64, k)[:] = int(q)
+        time.sleep(0.02)  # another thread runs here, as it does while the library searches
+        values(args.out_dists, ctypes.c_double, k)[:] = values(args.queries, ctypes.c_float, g.dim)[0]
+        values(args.out_counters, ctypes.c_int64, 2)[:] = ef
+        return 0
+
+    g.lib = SimpleNamespace(hnsw_b200_search=search)
+    got = {}
+
+    def work(i: int) -> None:
+        got[i] = g.search_one(np.full(8, float(i), dtype=np.float32), ks[i], 10 + i)
+
+    g.search_one(np.zeros(8, dtype=np.float32), 4, 10)  # the buffers are there before the threads are
+    _together(work, len(ks))
+    for i, (ids, dists, ctr) in got.items():
+        np.testing.assert_array_equal(ids, np.full(ks[i], i))
+        np.testing.assert_array_equal(dists, np.full(ks[i], float(i)))
+        np.testing.assert_array_equal(ctr, np.full(2, 10 + i))
