@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "hnsw_b200.h"
+#include "scratch.cuh"
 
 namespace hb {
 int fail(int code, const std::string &msg);  // search.cu: records the thread's last error
@@ -1256,25 +1257,22 @@ int make_map(CUtensorMap *map, const void *base, int64_t rows, int kpad, int box
     return 0;
 }
 
-struct Scratch {
-    void *p = nullptr;
-    size_t bytes = 0;
-    ~Scratch() {
-        if (p) cudaFree(p);
+struct CudaMem {
+    static bool device(int *d) { return cudaGetDevice(d) == cudaSuccess; }
+    static bool alloc(void **p, size_t bytes) {
+        if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+        cudaGetLastError();
+        return false;
     }
-    int get(size_t b) {
-        if (b <= bytes) return 0;
-        if (p) cudaFree(p);
-        p = nullptr;
-        bytes = 0;
-        if (cudaMalloc(&p, b) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(HNSW_B200_ENOMEM, "exact knn scratch allocation failed");
-        }
-        bytes = b;
-        return 0;
+    static void release(int d, void *p) {
+        int now = d;
+        cudaGetDevice(&now);
+        if (now != d) cudaSetDevice(d);
+        cudaFree(p);
+        if (now != d) cudaSetDevice(now);
     }
 };
+using Scratch = DeviceScratch<CudaMem>;
 
 #define XT(expr)                                                                               \
     do {                                                                                       \
@@ -1352,8 +1350,8 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
         bytes = bytes_ok;
     } else if (integer != 0) {  // find out on the device, one pass over each array
         static thread_local Scratch flag_buf;
-        if (int rc = flag_buf.get(16)) return rc;
-        int32_t *flag = static_cast<int32_t *>(flag_buf.p);
+        int32_t *flag = static_cast<int32_t *>(flag_buf.get(16));
+        if (!flag) return fail(HNSW_B200_ENOMEM, "exact knn scratch allocation failed");
         XT(cudaMemsetAsync(flag, 0, 4, s));
         check_small_int<<<1024, 256, 0, s>>>(static_cast<const float *>(a->data), n * dim, flag);
         check_small_int<<<256, 256, 0, s>>>(static_cast<const float *>(a->queries), nq_all * dim, flag);
@@ -1450,8 +1448,8 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
     const size_t o_ci = carve(size_t(slots) * cap * 4);
     const size_t o_st = carve(sizeof(Stats));
     const size_t o_mx = carve(16);
-    if (int rc = buf.get(off)) return rc;
-    char *B = static_cast<char *>(buf.p);
+    char *B = static_cast<char *>(buf.get(off));
+    if (!B) return fail(HNSW_B200_ENOMEM, "exact knn scratch allocation failed");
     auto *xb = reinterpret_cast<__nv_bfloat16 *>(B + o_xb);
     auto *qb = reinterpret_cast<__nv_bfloat16 *>(B + o_qb);
     auto *xn = reinterpret_cast<double *>(B + o_xn);
