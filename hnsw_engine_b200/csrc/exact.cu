@@ -1089,7 +1089,9 @@ __global__ void rerank_topk(const T *data, const T *queries, int dim, int32_t nq
                 d = dist_f64_lane(data + int64_t(id) * dim, qv, dim, metric, cos ? xnorm[id] : 1.0, qn);
             }
             if (need) err = fmax(err, fabs(double(approx) - d));
-            uint32_t am = __ballot_sync(0xffffffffu, has);
+            // Once there are k results, only candidates below the last go on, told by their lanes together; the
+            // last only comes nearer, so each is tested again at its turn.
+            uint32_t am = __ballot_sync(0xffffffffu, has && (a < k || pair_lt(d, id, Ad[k - 1], Ai[k - 1])));
             while (am) {
                 const int j = __ffs(am) - 1;
                 am &= am - 1;
@@ -1097,7 +1099,11 @@ __global__ void rerank_topk(const T *data, const T *queries, int dim, int32_t nq
                 const int32_t xi = __shfl_sync(0xffffffffu, id, j);
                 if (a == k && !pair_lt(xd, xi, Ad[k - 1], Ai[k - 1])) continue;
                 int c = 0;
-                for (int r = lane; r < a; r += 32) c += pair_lt(Ad[r], Ai[r], xd, xi);
+                if (!isnan(xd)) {
+                    for (int r = lane; r < a; r += 32) c += below(Ad[r], Ai[r], xd, xi);
+                } else {
+                    for (int r = lane; r < a; r += 32) c += pair_lt(Ad[r], Ai[r], xd, xi);
+                }
                 const int pos = __reduce_add_sync(0xffffffffu, c);
                 for (int top = a - 1; top >= pos; top -= 32) {
                     const int r = top - lane;

@@ -115,3 +115,29 @@ def test_zero_rows_and_queries_under_cosine_come_last(dim: int, n: int, k: int) 
         assert (norms[ids[i, m:]] == 0).all() and (norms[ids[i, :m]] > 0).all()
         _, w_d = _cosine_nan_last(data[norms > 0], queries[i : i + 1], max(m, 1))
         np.testing.assert_allclose(dists[i, :m], w_d[0, :m], rtol=0, atol=dim * 2.0**-52)
+
+
+@pytest.mark.parametrize("dim", [24, 300])
+@pytest.mark.parametrize("k", [1, 40, 3_000])
+def test_more_ties_than_are_gathered(dim: int, k: int) -> None:
+    """All rows but a few zero ones at one distance from the query, some just below it: results are inserted,
+    and rows at the last result's distance stay out unless their id is lower."""
+    import torch
+
+    from hnsw_engine_b200.exact_knn import exact_search
+
+    n = 6_000
+    rng = np.random.default_rng(dim)
+    data = np.zeros((n, dim), dtype=np.float32)
+    data[:, 0], data[:, 1] = 3.0, 4.0
+    near = rng.permutation(n)[:25]  # in no order of ids
+    data[near, 1] = np.linspace(3.0, 3.9, 25).astype(np.float32)
+    zero = rng.permutation(np.setdiff1d(np.arange(n), near))[:50]
+    data[zero] = 0.0
+    queries = np.zeros((2, dim), dtype=np.float32)
+    queries[0, 0] = 1.0
+    queries[1, 1] = 2.0
+    ids, dists = exact_search(torch.from_numpy(data).cuda(), torch.from_numpy(queries).cuda(), k, "cosine")
+    w_ids, w_d = _cosine_nan_last(data, queries, k)
+    np.testing.assert_array_equal(ids.cpu().numpy(), w_ids)
+    np.testing.assert_allclose(dists.cpu().numpy(), w_d, rtol=0, atol=dim * 2.0**-52)
