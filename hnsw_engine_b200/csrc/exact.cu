@@ -777,15 +777,16 @@ constexpr int SELECT_WARPS = 8;
 // final_pass: the list is pass two's, out_tau holds the threshold it was collected with (without the
 // margin), and *short_lists is set when that threshold turns out too low: fewer than k entries, or
 // a k-th smallest above it. stat_max: largest |value| the error bound is stated for (byte rows: the
-// finite final thresholds; else the margins), as float bits.
+// finite final thresholds; else the margins), as float bits. longest (final pass): the longest segment count;
+// where lists overflowed the call runs again, and nothing here is worth doing.
 __global__ void select_kth(float *cand_val, int32_t *cand_id, const int32_t *cand_cnt, int32_t cap,
                            int32_t nseg, int32_t nq, int32_t k, const float *margin, float *out_thr,
                            float *out_tau, int32_t *cand_m, int final_pass, int bytes,
-                           int32_t *short_lists, unsigned int *stat_max) {
+                           int32_t *short_lists, unsigned int *stat_max, const unsigned long long *longest) {
     __shared__ uint32_t hist_all[SELECT_WARPS][256];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q = blockIdx.x * SELECT_WARPS + wid;
-    if (q >= nq) return;  // no block-wide barrier below
+    if (q >= nq || (longest && *longest > static_cast<unsigned long long>(cap))) return;  // no block-wide barrier below
     uint32_t *hist = hist_all[wid];
     float *v = cand_val + int64_t(q) * nseg * cap;
     const int m = compact_list(v, cand_id ? cand_id + int64_t(q) * nseg * cap : nullptr,
@@ -971,17 +972,22 @@ __host__ __device__ inline size_t rerank_smem(int k, int dim, bool gather, bool 
 // position) is re-scored in float64 at the end instead, and any difference sets *mismatch. (Re-scoring every query's results cost 0.55 ms of 8.6 on the 1M x 128 mixture and
 // 0.63 of 2.6 on the 60K x 784 set, 10K queries each; integer products and sums are exact, so
 // the check is there to catch a wrong operand layout or descriptor, which a sample shows.)
+// longest, short_lists (NULL: not looked at): as for select_kth; lists that overflowed or came from too low a
+// threshold are collected again, and their results would be thrown away. 10K queries x 1M x 128 bytes in runs of
+// 1,000 similar rows, k = 100: 12.9 -> 12.4 ms; 2,000 x 60K x 784 floats in runs of 600: 3.77 -> 2.84 ms.
 template <typename T>
 __global__ void rerank_topk(const T *data, const T *queries, int dim, int32_t nq, int32_t k,
                             int32_t metric, const double *xnorm, const double *qnorm,
                             const float *cand_val, const int32_t *cand_id, const int32_t *cand_m,
                             int32_t cap, int32_t nseg, const float *thr, int64_t *out_ids,
                             double *out_d, unsigned long long *err_max, float exact_lim,
-                            int32_t *mismatch, int gather, int products) {
+                            int32_t *mismatch, int gather, int products, const unsigned long long *longest,
+                            const int32_t *short_lists) {
     extern __shared__ __align__(16) unsigned char sm[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q = blockIdx.x * (blockDim.x >> 5) + w;
-    if (q >= nq) return;  // no block-wide barrier below
+    if (q >= nq || *longest > static_cast<unsigned long long>(cap) || (short_lists && *short_lists))
+        return;  // no block-wide barrier below
     const int slots = gather ? survivor_slots(k) : 0;
     unsigned char *base = sm + size_t(w) * rerank_smem(k, dim, gather, products);
     double *Ad = reinterpret_cast<double *>(base);       // results
@@ -1297,7 +1303,7 @@ constexpr int64_t MAX_CHUNK = 16384;  // queries of a batch filtered together
 // segment. With half a tile's columns of slack (32) such rows overflowed and the call ran twice: 10K
 // queries x 1M x 128 bytes in 10,000 runs of similar rows, k = 100, 8.36 -> 4.20 ms; 2,000 x 200K x 64 floats
 // in 10,000 runs, k = 10, 936 -> 480 us; rows in no order take the same time with either (3.21 ms,
-// 430 us). Longer runs still overflow (1,000 rows each: 12.6 ms).
+// 430 us). Longer runs still overflow (1,000 rows each: 12.4 ms).
 constexpr int64_t SEGMENT_FACTOR = 6;
 constexpr int64_t SEGMENT_SLACK = 4 * CW;
 // Byte rows use the integer filter (1) or the BF16 one (0).
@@ -1582,7 +1588,7 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
             const int sel_blocks = int((nq + SELECT_WARPS - 1) / SELECT_WARPS);
             select_kth<<<sel_blocks, 32 * SELECT_WARPS, 0, s>>>(
                 cv, nullptr, cnt, int32_t(cap), int32_t(nseg), int32_t(nq), pass_rank, mg, th, tau, cm, 0,
-                bytes, nullptr, nullptr);
+                bytes, nullptr, nullptr, nullptr);
             // Pass two: every row against tau + margin; the k-th smallest candidate is the global
             // k-th approximate distance, the final threshold.
             if (int rc = run_filter(tiles, 1, th, false)) return rc;
@@ -1590,11 +1596,12 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
                 cnt, nq * nseg, &st->longest);
             select_kth<<<sel_blocks, 32 * SELECT_WARPS, 0, s>>>(
                 cv, ci, cnt, int32_t(cap), int32_t(nseg), int32_t(nq), k, mg, th, tau, cm, 1, bytes,
-                &st->short_lists, &st->bound);
+                &st->short_lists, &st->bound, &st->longest);
             rerank_topk<T><<<int((nq + wpb - 1) / wpb), wpb * 32, rsm, s>>>(
                 X, Q, dim, int32_t(nq), k, metric, xn, qn, cv, ci, cm, int32_t(cap), int32_t(nseg), th,
                 a->out_ids + q0 * k, a->out_dists + q0 * k, &st->filter_err, bytes ? EXACT_LIM : 0.f,
-                &st->mismatch, gather, gather && products);
+                &st->mismatch, gather, gather && products, &st->longest,
+                pass_rank == k ? nullptr : &st->short_lists);
             XT(cudaGetLastError());
             launches += 4;
             XT(cudaMemcpyAsync(&hst, st, sizeof(Stats), cudaMemcpyDeviceToHost, s));

@@ -141,3 +141,26 @@ def test_more_ties_than_are_gathered(dim: int, k: int) -> None:
     w_ids, w_d = _cosine_nan_last(data, queries, k)
     np.testing.assert_array_equal(ids.cpu().numpy(), w_ids)
     np.testing.assert_allclose(dists.cpu().numpy(), w_d, rtol=0, atol=dim * 2.0**-52)
+
+
+@pytest.mark.parametrize("as_bytes", [True, False])
+@pytest.mark.parametrize("run,k", [(1_000, 10), (10_000, 10), (10_000, 300)])
+def test_lists_that_overflow_are_collected_again(as_bytes: bool, run: int, k: int) -> None:
+    """Rows in runs longer than a segment has room for: the first attempt is thrown away, and the next one's
+    results are whole."""
+    import torch
+
+    from hnsw_engine_b200.exact_knn import exact_search
+
+    rng = np.random.default_rng(run + k)
+    n, dim, nq = 100_000, 24, 140
+    centres = rng.random((n // run, dim)) * 128 + 30
+    data = centres[np.sort(rng.integers(0, n // run, n))] + 20 * rng.standard_normal((n, dim))
+    queries = centres[rng.integers(0, n // run, nq)] + 20 * rng.standard_normal((nq, dim))
+    if as_bytes:
+        data, queries = np.rint(data).clip(0, 255), np.rint(queries).clip(0, 255)
+    data, queries = data.astype(np.float32), queries.astype(np.float32)
+    ids, dists = exact_search(torch.from_numpy(data).cuda(), torch.from_numpy(queries).cuda(), k, "l2")
+    o_ids, o_d = exact.exact_search(data, queries, k, "l2")
+    np.testing.assert_array_equal(ids.cpu().numpy(), o_ids)
+    np.testing.assert_allclose(dists.cpu().numpy(), o_d, rtol=0 if as_bytes else dim * 2.0**-52)
