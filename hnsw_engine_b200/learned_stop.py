@@ -38,6 +38,9 @@ from .engine import DeviceGraph, to_device
 from .metrics import RELATIVE_TIE_TOLERANCE
 
 FEATURES = 12
+# Samples that training gathers at once (200 MB of features): one gather for most epochs, and no second copy of
+# a training set of any size.
+GATHER_SAMPLES = 1 << 22
 HIDDEN = 64
 STOP_EVERY = 16
 FEATURE_NAMES = (
@@ -189,10 +192,14 @@ class StopNetwork:
                 order = torch.randperm(n, generator=g).to(self.device)
                 ep_loss, nb = 0.0, 0
                 rate = lr * (0.5 ** ep)
-                used = order[: n // batch * batch]  # the epoch's samples in its order, gathered once
-                Xe, ye = Xd[used], yd[used]
+                used = n // batch * batch
+                piece = max(batch, GATHER_SAMPLES // batch * batch)
                 for s in range(0, n - batch + 1, batch):
-                    xb, yb = Xe[s : s + batch], ye[s : s + batch]
+                    at = s % piece
+                    if at == 0:  # the next samples in the epoch's order, gathered together
+                        part = order[s : min(s + piece, used)]
+                        Xe, ye = Xd[part], yd[part]
+                    xb, yb = Xe[at : at + batch], ye[at : at + batch]
                     self.step += 1
                     _lib.check(self.lib.hnsw_b200_mlp_train_step(
                         _ptr(self.params), _ptr(self.m), _ptr(self.v), self.step, rate, _ptr(xb),
