@@ -334,7 +334,8 @@ void launch_step(const float *params, const float *features, const float *target
     mlp_grads<<<GRAD_BLOCKS, GRAD_THREADS, smem, s>>>(features, H1, H2, dH1, dH2, dO, batch, G, A);
 }
 
-size_t scratch_floats(int B) { return size_t(B) * (4 * H + 1) + NPARAM + 4; }
+// H1, H2, dH1, dH2 and dO (launch_step)
+size_t scratch_floats(int B) { return size_t(B) * (4 * H + 1); }
 
 }  // namespace hbm
 
