@@ -34,6 +34,7 @@
 
 #include "hnsw_b200.h"
 #include "scratch.cuh"
+#include "split.cuh"
 
 namespace hb {
 int fail(int code, const std::string &msg);  // search.cu: records the thread's last error
@@ -1384,28 +1385,8 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
 
-    // Split geometry of a pass over `tiles` tiles for a chunk of nqc queries: a CTA takes tps tiles of
-    // one query tile, and the split is the one whose waves of CTAs (one an SM) end soonest, a CTA's
-    // start and end counted as FIXED_TILES tiles.
-    constexpr int FIXED_TILES = 3;
-    struct Geo {
-        int tps, splits;
-    };
-    auto geo = [&](int64_t nqc, int tiles) {
-        const int qt = int((nqc + BM - 1) / BM);
-        const int most = std::min(tiles, std::max(1, (8 * sms + qt - 1) / qt));
-        Geo g{tiles, 1};
-        int64_t best = INT64_MAX;
-        for (int s = 1; s <= most; s++) {
-            const int tps = (tiles + s - 1) / s, splits = (tiles + tps - 1) / tps;
-            const int64_t waves = (int64_t(qt) * splits + sms - 1) / sms, cost = waves * (tps + FIXED_TILES);
-            if (cost < best) {
-                best = cost;
-                g = Geo{tps, splits};
-            }
-        }
-        return g;
-    };
+    // Split of a pass over `tiles` tiles for a chunk of nqc queries.
+    auto geo = [&](int64_t nqc, int tiles) { return split_tiles(int((nqc + BM - 1) / BM), tiles, sms); };
     // Pass one keeps the minimum of every block of two tiles' chunks of an epilogue thread (every row when
     // the sample has fewer than k blocks); pass two keeps the rows within tau + margin. Each epilogue
     // thread appends to its own segment of the query's list: in pass one at most one entry per block
@@ -1426,7 +1407,7 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
         cap = slots = 0;
         const int64_t last = nq_all % QB ? nq_all % QB : QB;
         for (int64_t nqc : {QB, last}) {
-            const Geo g1 = geo(nqc, sample), g2 = geo(nqc, tiles);
+            const Split g1 = geo(nqc, sample), g2 = geo(nqc, tiles);
             const int64_t nseg2 = int64_t(g2.splits) * EPI_PER_QUARTER;
             const int64_t share = (SEGMENT_FACTOR * expect2 + nseg2 - 1) / nseg2 + SEGMENT_SLACK;
             cap = std::max<int64_t>(cap, block_min ? (g1.tps + 1) / 2 : int64_t(2 * CW) * g1.tps);
@@ -1547,7 +1528,7 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
         const int qt_chunk = int((nq + BM - 1) / BM);
         int nseg = 0;  // segments per query of the last pass run
         auto run_filter = [&](int pass_tiles, int pass_stride, const float *pass_thr, bool bmin) -> int {
-            const Geo gg = geo(nq, pass_tiles);
+            const Split gg = geo(nq, pass_tiles);
             nseg = gg.splits * EPI_PER_QUARTER;
             FilterParams fp;
             fp.nq = int32_t(nq);
