@@ -231,7 +231,7 @@ struct SearchParams {
     int32_t trace_cap;
     int32_t trace_k;        // distances recorded per checkpoint (min(k, 16))
     int32_t lane_rows;      // byte rows may use mark_score_lane_rows (see the host's choice)
-    int32_t code_rows;      // rows of a tile of code_chunk_dists, or 0 (see code_tile_choice)
+    int32_t code_rows;      // rows of a tile of code_chunk_dists (24 or 16), or 0 (see code_tile_choice)
 };
 
 constexpr int STOP_EVERY = 16;
@@ -2414,13 +2414,25 @@ int occupancy(int mode, bool u8, bool filt, int cfg, size_t smem_block, int *bps
               : occupancy_cfg<0, false, 0>(filt, smem_block, bps);
 }
 
-// The rows of code_chunk_dists' tiles: the most with which as many blocks stay resident as without (24 cover
-// most chunks in one pass; at large ef the results leave less room), or 0, where a lane reads its own row: no
-// room, or rows that do not start on 4-byte boundaries.
+// The rows of code_chunk_dists' tiles: 24, which cover most chunks in one pass, or 16, where as many blocks stay
+// resident as without; or 0, where a lane reads its own row. A tile takes an instruction a row and 128 bytes
+// whatever part of them the row fills, and a pass takes its sums' time however few rows it has; a lane's own loads
+// touch a row's sectors once when it starts on one, and about twice when it does not. Time over that of a lane a
+// row (20K to 300K rows of normal or heavy-tailed data, ef 50 to 400, one query / 3,000):
+//   widths off 32 bytes: 24 rows, 36 to 52 codes 0.81 to 1.05 / 0.88 to 1.12, 68 to 228 codes 0.61 to 1.04 /
+//     0.73 to 1.06; 16 rows, where 24 do not fit, 68 to 228 codes 0.59 to 1.01 / 0.77 to 1.10;
+//   whole pieces: 24 rows, 128 codes 0.87 to 1.10 / 0.86 to 0.95, 256 codes 0.98 / 0.86; 16 rows up to 1.14;
+//   other multiples of 32: 64 codes 1.06 / 1.12, 96 codes 1.09 to 1.14 / 1.14 to 1.16, 160 codes 1.12 / 1.21;
+//   at most 32 codes: 1.02 to 1.17 / 1.04 to 1.23;
+//   8 rows: 128 codes 1.2 to 1.6, 256 codes 1.5, 100 codes 0.9 to 1.2 (before there were tiles, a lane a row with
+//     the admission of that time took about 1.1).
 int code_tile_choice(int mode, bool u8, bool filt, int dim, size_t *smem_block, int *bps, int *rows) {
     *rows = 0;
     if (mode != MODE_F64 || !u8 || (dim & 3) != 0) return 0;
-    for (int r : {24, 16, 8}) {
+    const bool sectors = dim % 32 == 0;
+    if (dim <= 32 || (sectors && dim % 128 != 0)) return 0;
+    for (int r : {24, 16}) {
+        if (sectors && r < 24) break;
         const size_t with = *smem_block + WPB * code_tile_bytes(r);
         if (with > 227 * 1024) continue;
         int b = 0;

@@ -65,3 +65,20 @@ def test_byte_rows_match_the_oracle(dim: int, metric: str) -> None:
         np.testing.assert_array_equal(ids.cpu().numpy(), o_ids)
         np.testing.assert_array_equal(dists.cpu().numpy(), o_d)
         np.testing.assert_array_equal(ctr.cpu().numpy(), o_c)
+
+
+# Around the widths and result capacities at which code rows go through tiles of 24 rows, of 16, or none: up to 32
+# codes and multiples of 32 that fill no whole pieces (none), others (by the room that ef leaves).
+@pytest.mark.parametrize("dim,ef", [(28, 24), (32, 24), (36, 350), (64, 24), (96, 60), (100, 24), (100, 350), (100, 550),
+                                    (128, 350), (160, 24), (256, 24), (256, 200), (384, 24)])
+@pytest.mark.parametrize("metric", ["l2", "cosine"])
+def test_code_rows_match_the_oracle_where_tiles_change(dim: int, ef: int, metric: str) -> None:
+    from oracle import cpu
+
+    index, arrays, ep, ml, codes = _codes_case(dim, metric)
+    queries = np.random.default_rng(2).standard_normal((12, dim)) * 100 + 120
+    ids, dists, ctr = index.device_graph.search(queries, 10, ef, use_codes=True)
+    o_ids, o_d, o_c = cpu.search_batch(arrays, ep, ml, queries, 10, ef, metric, codes=codes, threads=8)
+    np.testing.assert_array_equal(ids.cpu().numpy(), o_ids)
+    np.testing.assert_array_equal(dists.cpu().numpy(), o_d)
+    np.testing.assert_array_equal(ctr.cpu().numpy(), o_c)
