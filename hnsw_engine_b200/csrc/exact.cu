@@ -89,6 +89,8 @@ struct FilterParams {
     int32_t stages;        // operand stages in flight
     int32_t a_resident;    // the query tile's operand is loaded once and stays (else with each stage)
     int32_t tiles_per_split;
+    int32_t tile_blocks;   // threshold pass: blocks of an epilogue thread's part of a tile: 1, 2, 4, 8 or 16 (groups
+                           // of four rows); 0: a block is the thread's part of two tiles
     int32_t metric;
     const float *qq;       // |q|^2 per query (l2)
     const float *xx;       // per row: |x|^2 (l2) or 0; +inf past the data rows
@@ -290,6 +292,14 @@ struct EpiThread {
                          value(r[4 * g + 3], x.w));
         }
         return min3(min3(min3(mg[0], mg[1], mg[2]), mg[3], mg[4]), min2(mg[5], mg[6]), mg[7]);
+    }
+
+    // Threshold pass: keeps the first `count` of the block minima m.
+    __device__ __forceinline__ void keep(const V (&m)[CW / 4], int count) {
+#pragma unroll
+        for (int g = 0; g < CW / 4; g++)
+            if (g < count && cnt + g < cap) cv[cnt + g] = float(m[g] + add);
+        cnt += count;
     }
 
     // Appends the chunk's candidates: of the groups of four that hold one for some query of the warp,
@@ -559,11 +569,16 @@ __global__ void __launch_bounds__(FILTER_THREADS, 1)
             const unsigned char *xslot = xring + (lt % XSLOTS) * BN * 4;
             const int valid0 = p.row_end - row0 - c0, valid1 = p.row_end - row0 - c1;
             uint32_t r0[CW], r1[CW];
-            typename EpiThread<I8>::V mg[CW / 4];
+            typename EpiThread<I8>::V mg[CW / 4], bmg[CW / 4];
             tmem_ld(tbase + uint32_t(c0), r0);
             tmem_wait(r0);
             tmem_ld(tbase + uint32_t(c1), r1);  // in flight while the first chunk is worked on
             const auto m0 = E.minima(r0, xslot + c0 * 4, mg);
+            if constexpr (BMIN) {
+                if (p.tile_blocks == 16 && qvalid) E.keep(mg, 8);
+#pragma unroll
+                for (int g = 0; g < CW / 4; g++) bmg[g] = mg[g];
+            }
             if (!BMIN && __any_sync(0xffffffffu, E.pass(m0)))
                 E.append(tbase + uint32_t(c0), xslot + c0 * 4, row0 + c0, valid0, mg);
             tmem_wait(r1);
@@ -576,16 +591,30 @@ __global__ void __launch_bounds__(FILTER_THREADS, 1)
                 mbar_arrive(tempty + b);
                 mbar_arrive(xempty + lt % XSLOTS);
             }
-            // Threshold pass: one value per block, the minimum of this thread's chunks of two tiles. The
-            // r-th smallest of the blocks' minima is at least the r-th smallest of all the values (a
-            // subset's r-th is never below the set's); with far more blocks than r it is nearly as tight.
-            // Values only: the pass needs no row ids.
+            // Threshold pass: one value per block, its minimum. The r-th smallest of the blocks' minima is at
+            // least the r-th smallest of all the values (a subset's r-th is never below the set's), and nearly as
+            // tight where there are at least twice as many blocks (see tile_blocks at the host). Values only: the
+            // pass needs no row ids.
             if constexpr (BMIN) {
-                const auto m = min2(m0, m1);
-                bm = b == 0 ? m : min2(bm, m);
-                if ((b == 1 || lt + 1 == ntiles) && qvalid) {
-                    if (E.cnt < E.cap) E.cv[E.cnt] = float(bm + E.add);
-                    E.cnt++;
+                if (p.tile_blocks == 16) {
+                    if (qvalid) E.keep(mg, 8);
+                } else {
+#pragma unroll
+                    for (int g = 0; g < 8; g++) bmg[g] = min2(bmg[g], mg[g]);
+                    if (p.tile_blocks <= 4) {
+#pragma unroll
+                        for (int g = 0; g < 4; g++) bmg[g] = min2(bmg[g], bmg[g + 4]);
+                    }
+                    if (p.tile_blocks <= 2) {
+                        bmg[0] = min2(bmg[0], bmg[2]);
+                        bmg[1] = min2(bmg[1], bmg[3]);
+                    }
+                    if (p.tile_blocks <= 1) bmg[0] = min2(bmg[0], bmg[1]);
+                    if (p.tile_blocks == 0) {  // the part of two tiles
+                        bmg[0] = b == 0 ? bmg[0] : min2(bm, bmg[0]);
+                        bm = bmg[0];
+                    }
+                    if (qvalid && (p.tile_blocks > 0 || b == 1 || lt + 1 == ntiles)) E.keep(bmg, max(1, p.tile_blocks));
                 }
             }
         }
@@ -1387,9 +1416,8 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
 
     // Split of a pass over `tiles` tiles for a chunk of nqc queries.
     auto geo = [&](int64_t nqc, int tiles) { return split_tiles(int((nqc + BM - 1) / BM), tiles, sms); };
-    // Pass one keeps the minimum of every block of two tiles' chunks of an epilogue thread (every row when
-    // the sample has fewer than k blocks); pass two keeps the rows within tau + margin. Each epilogue
-    // thread appends to its own segment of the query's list: in pass one at most one entry per block
+    // Pass one keeps the minimum of every block of rows (tile_blocks), or every row where the sample has fewer than
+    // 4 k; pass two keeps the rows within tau + margin. Each epilogue thread appends to its own segment of the query's list: in pass one at most one entry per block
     // or its 2 CW columns of a tile; pass two's segments get SEGMENT_FACTOR times their even share of the
     // expected candidates and SEGMENT_SLACK more, and never more than the columns that they cover (an
     // overflow re-runs the call with longer segments).
@@ -1398,7 +1426,15 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
         n, std::max<int64_t>(int64_t(64) * k, int64_t(std::sqrt(SAMPLE_BALANCE * double(k) * double(n)))));
     const int stride = std::max<int>(1, int(tiles / ((sample_rows + BN - 1) / BN)));
     const int sample = (tiles + stride - 1) / stride;  // tiles 0, stride, 2 stride, ... of pass one
-    const bool block_min = int64_t(sample) / 2 * EPI_PER_QUARTER >= k;
+    const int64_t pad = int64_t(sample - 1) * stride == tiles - 1 ? n_pad - n : 0;  // of the last sampled tile
+    const int64_t whole = sample - (pad > 0), sampled = int64_t(sample) * BN - pad;
+    // The largest blocks of which the sample surely has 2 k: k ln 4 rows of it lie below the k-th smallest of 2 k
+    // minima, and fewer blocks make a looser threshold (1,000 rows' k-th of k minima is their largest) while every
+    // row kept makes pass one append, which takes ten times as long (200 queries x 700 rows, k = 10: 68 us of a
+    // call's 225).
+    int tile_blocks = int64_t(sample) / 2 * EPI_PER_QUARTER >= 2 * int64_t(k) ? 0 : 1;
+    while (tile_blocks > 0 && tile_blocks < 16 && whole * EPI_PER_QUARTER * tile_blocks < 2 * int64_t(k)) tile_blocks *= 2;
+    const bool block_min = tile_blocks < 16 || sampled / 4 >= k;
     const int rank = sample_rank(k, sample, tiles);
     const int64_t expect2 = int64_t(rank) * tiles / sample + int64_t(k) / 2;  // candidates of a query
     int64_t QB = std::min<int64_t>(nq_all, MAX_CHUNK);  // queries per chunk
@@ -1410,7 +1446,7 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
             const Split g1 = geo(nqc, sample), g2 = geo(nqc, tiles);
             const int64_t nseg2 = int64_t(g2.splits) * EPI_PER_QUARTER;
             const int64_t share = (SEGMENT_FACTOR * expect2 + nseg2 - 1) / nseg2 + SEGMENT_SLACK;
-            cap = std::max<int64_t>(cap, block_min ? (g1.tps + 1) / 2 : int64_t(2 * CW) * g1.tps);
+            cap = std::max<int64_t>(cap, !block_min ? int64_t(2 * CW) * g1.tps : tile_blocks ? int64_t(tile_blocks) * g1.tps : (g1.tps + 1) / 2);
             cap = std::max<int64_t>(cap, std::min<int64_t>(std::max(cap_min, share), int64_t(2 * CW) * g2.tps));
             slots = std::max<int64_t>(slots, nqc * std::max(g1.splits, g2.splits) * EPI_PER_QUARTER);
         }
@@ -1539,6 +1575,7 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
             fp.stages = nstages;
             fp.a_resident = resident ? 1 : 0;
             fp.tiles_per_split = gg.tps;
+            fp.tile_blocks = tile_blocks;
             fp.metric = metric;
             fp.qq = qq;
             fp.xx = xx;
