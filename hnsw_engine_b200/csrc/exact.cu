@@ -916,43 +916,6 @@ __device__ __forceinline__ double dist_f64_lane(const T *x, const T *qv, int dim
     return __dsub_rn(1.0, acc);
 }
 
-// Float64 distances of up to 32 rows (ids[0 .. m) in shared memory) with the same sums in dimension
-// order: the warp computes the products of 32 dimensions of every row together (coalesced loads; under
-// cosine the two divisions of each product, which are most of the work, spread over the lanes), then
-// lane s adds row s's products in order. qs: the query's values (cosine: divided by its norm) in
-// shared memory; P: 32 rows of DIST_PITCH doubles. Lane s < m returns its row's distance.
-constexpr int DIST_PITCH = 33;
-template <typename T>
-__device__ __forceinline__ double dist_f64_rows(const T *data, const int32_t *ids, int m, const double *qs,
-                                                int dim, int metric, const double *xnorm, double *P,
-                                                int lane) {
-    double acc = 0.0;
-    for (int d0 = 0; d0 < dim; d0 += 32) {
-        const int d = d0 + lane;
-        const double qd = d < dim ? qs[d] : 0.0;
-        for (int s = 0; s < m; s++) {
-            const int64_t id = ids[s];
-            double pr = 0.0;
-            if (d < dim) {
-                const double x = double(data[id * dim + d]);
-                if (metric == HNSW_B200_L2) {
-                    const double df = __dsub_rn(x, qd);
-                    pr = __dmul_rn(df, df);
-                } else {
-                    pr = __dmul_rn(metric == HNSW_B200_IP ? x : __ddiv_rn(x, xnorm[id]), qd);
-                }
-            }
-            P[s * DIST_PITCH + lane] = pr;
-        }
-        __syncwarp();
-        const int nd = min(32, dim - d0);
-        if (lane < m)
-            for (int j = 0; j < nd; j++) acc = __dadd_rn(acc, P[lane * DIST_PITCH + j]);
-        __syncwarp();
-    }
-    return metric == HNSW_B200_L2 ? acc : (metric == HNSW_B200_IP ? -acc : __dsub_rn(1.0, acc));
-}
-
 // The same by the whole warp (long rows): lane l sums dimensions l, l + 32, ..., then a fixed
 // shuffle tree adds the lanes (the same value on every run; on integer data every order gives the
 // same exact sum), so the float64 chains are 32 times shorter. The result is on every lane.
@@ -979,13 +942,9 @@ __device__ __forceinline__ double dist_f64_warp(const T *x, const T *qv, int dim
 // Survivors (candidates within the final threshold) of a query that rerank_topk gathers in shared
 // memory and sorts there; a query with more (many exact ties) inserts them one by one.
 __host__ __device__ constexpr int survivor_slots(int k) { return k + k / 4 + 64; }
-// Shared memory of one warp of rerank_topk: distances and ids of the results and of the survivors,
-// then (rows below COOP_DIM re-scored in float64) the query and a block of products.
-__host__ __device__ inline size_t rerank_smem(int k, int dim, bool gather, bool products) {
-    size_t b = size_t(k + 1 + (gather ? survivor_slots(k) : 0)) * 12;
-    b = (b + 15) & ~size_t(15);
-    if (products) b += size_t(dim) * 8 + size_t(32) * DIST_PITCH * 8;
-    return (b + 15) & ~size_t(15);
+// Shared memory of one warp of rerank_topk: distances and ids of the results and of the survivors.
+__host__ __device__ inline size_t rerank_smem(int k, bool gather) {
+    return (size_t(k + 1 + (gather ? survivor_slots(k) : 0)) * 12 + 15) & ~size_t(15);
 }
 
 // One warp per query: exact float64 distances of the candidates within the final threshold,
@@ -993,9 +952,8 @@ __host__ __device__ inline size_t rerank_smem(int k, int dim, bool gather, bool 
 // gather: the survivors are first collected in shared memory (most candidates fail the final threshold:
 // scored in batches of candidates, a float64 chain ran for one or two of 32 lanes), scored 32 at a
 // time and placed by counting the ones below each: about k^2 / 32 steps, against k insertions of about 80
-// instructions. 10K queries x 1M x 128 bytes, k = 100: 332 -> 102 us; 1,000 x 200K x 100 cosine,
-// k = 10: 156 -> 33 us. Without room (k of several thousand) or with more survivors than slots
-// (ties), sorted insertion.
+// instructions. 10K queries x 1M x 128 bytes, k = 100: 332 -> 102 us. Where the slots would leave too few warps
+// (the host's choice) or with more survivors than slots (ties), sorted insertion.
 // exact_lim > 0 (byte rows, integer filter): a candidate whose filter value is below exact_lim in
 // magnitude already holds its exact distance and is not re-scored; one result in VERIFY_EVERY of
 // every query (positions q, q + VERIFY_EVERY, ... mod VERIFY_EVERY, so a batch covers every
@@ -1011,7 +969,7 @@ __global__ void rerank_topk(const T *data, const T *queries, int dim, int32_t nq
                             const float *cand_val, const int32_t *cand_id, const int32_t *cand_m,
                             int32_t cap, int32_t nseg, const float *thr, int64_t *out_ids,
                             double *out_d, unsigned long long *err_max, float exact_lim,
-                            int32_t *mismatch, int gather, int products, const unsigned long long *longest,
+                            int32_t *mismatch, int gather, const unsigned long long *longest,
                             const int32_t *short_lists) {
     extern __shared__ __align__(16) unsigned char sm[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1019,13 +977,11 @@ __global__ void rerank_topk(const T *data, const T *queries, int dim, int32_t nq
     if (q >= nq || *longest > static_cast<unsigned long long>(cap) || (short_lists && *short_lists))
         return;  // no block-wide barrier below
     const int slots = gather ? survivor_slots(k) : 0;
-    unsigned char *base = sm + size_t(w) * rerank_smem(k, dim, gather, products);
+    unsigned char *base = sm + size_t(w) * rerank_smem(k, gather);
     double *Ad = reinterpret_cast<double *>(base);       // results
     double *Sd = Ad + k + 1;                             // survivors
     int32_t *Ai = reinterpret_cast<int32_t *>(Sd + slots);
     int32_t *Si = Ai + k + 1;
-    double *qs = reinterpret_cast<double *>(base + rerank_smem(k, dim, gather, false));
-    double *P = qs + dim;
     const float t = thr[q];
     const T *qv = queries + int64_t(q) * dim;
     const bool cos = metric == HNSW_B200_COSINE;
@@ -1056,11 +1012,6 @@ __global__ void rerank_topk(const T *data, const T *queries, int dim, int32_t nq
         __syncwarp();
     }
     if (ns >= 0) {
-        if (products && !cos)
-            for (int i = lane; i < dim; i += 32) qs[i] = double(qv[i]);
-        if (products && cos)
-            for (int i = lane; i < dim; i += 32) qs[i] = __ddiv_rn(double(qv[i]), qn);
-        __syncwarp();
         for (int b0 = 0; b0 < ns; b0 += 32) {
             const int s = b0 + lane;
             const double approx = s < ns ? Sd[s] : 0.0;
@@ -1076,10 +1027,7 @@ __global__ void rerank_topk(const T *data, const T *queries, int dim, int32_t nq
                                                     cos ? xnorm[idj] : 1.0, qn, lane);
                     if (lane == j) d = dd;
                 }
-            } else if (products) {
-                const double dd = dist_f64_rows(data, Si + b0, min(32, ns - b0), qs, dim, metric, xnorm, P, lane);
-                if (need) d = dd;
-            } else if (need) {  // byte rows: distances of 2^24 or more only
+            } else if (need) {
                 d = dist_f64_lane(data + int64_t(Si[s]) * dim, qv, dim, metric, cos ? xnorm[Si[s]] : 1.0, qn);
             }
             if (need) {
@@ -1538,9 +1486,15 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
     const size_t smem = a_bytes + nstages * stage_bytes + XSLOTS * BN * 4 + 1024 + BAR_BYTES;
     const int wpb = 4;
     if (size_t(wpb) * (k + 1) * 12 > 200 * 1024) return fail(HNSW_B200_EINVAL, "k too large for the rerank kernel");
-    const bool products = !bytes && dim < COOP_DIM;
-    const bool gather = wpb * rerank_smem(k, dim, true, products) <= 200 * 1024;
-    const size_t rsm = wpb * rerank_smem(k, dim, gather, gather && products);
+    // Survivors are gathered where that leaves an SM two blocks of four queries (k up to about 1,000), under cosine
+    // nine (k up to about 210): a lane's divisions want many warps, which the insertion's smaller memory lets
+    // in. Time of a search with them gathered over inserted, 20K to 100K rows of 32 to 400 values, 100 to 10K
+    // queries: l2 and ip 0.67 to 1.14 up to k = 1,000 and 0.74 to 1.53 above, bytes 0.63 to 1.05 and 0.71 to
+    // 1.31, cosine 0.58 to 0.99 up to k = 200 and 0.69 to 1.77 above. (With the products of a batch's rows laid out in
+    // shared memory as well, cosine at k = 10 took the same time, and from k = 1,000 on up to 1.5 times the time
+    // without.)
+    const bool gather = wpb * rerank_smem(k, true) * (cos ? 9 : 2) <= size_t(SMEM_MAX);
+    const size_t rsm = wpb * rerank_smem(k, gather);
     XT(cudaFuncSetAttribute(rerank_topk<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(rsm)));
     XT(cudaMemsetAsync(st, 0, sizeof(Stats), s));
     Stats hst;
@@ -1618,7 +1572,7 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
             rerank_topk<T><<<int((nq + wpb - 1) / wpb), wpb * 32, rsm, s>>>(
                 X, Q, dim, int32_t(nq), k, metric, xn, qn, cv, ci, cm, int32_t(cap), int32_t(nseg), th,
                 a->out_ids + q0 * k, a->out_dists + q0 * k, &st->filter_err, bytes ? EXACT_LIM : 0.f,
-                &st->mismatch, gather, gather && products, &st->longest,
+                &st->mismatch, gather, &st->longest,
                 pass_rank == k ? nullptr : &st->short_lists);
             XT(cudaGetLastError());
             launches += 4;

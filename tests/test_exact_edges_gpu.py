@@ -164,3 +164,26 @@ def test_lists_that_overflow_are_collected_again(as_bytes: bool, run: int, k: in
     o_ids, o_d = exact.exact_search(data, queries, k, "l2")
     np.testing.assert_array_equal(ids.cpu().numpy(), o_ids)
     np.testing.assert_allclose(dists.cpu().numpy(), o_d, rtol=0 if as_bytes else dim * 2.0**-52)
+
+
+# k over the blocks of the threshold pass (two tiles, a tile's part, its halves to sixteenths, every row) and over the
+# sizes at which survivors are gathered (cosine about 210, else about 1,050).
+@pytest.mark.parametrize("k", [1, 10, 20, 50, 100, 200, 213, 400, 600, 1_040, 1_060])
+@pytest.mark.parametrize("kind", ["bytes", "l2", "ip", "cosine"])
+def test_results_at_every_size_of_block(kind: str, k: int) -> None:
+    import torch
+
+    from hnsw_engine_b200.exact_knn import exact_search
+
+    n, dim, nq = 2_000, 24, 70
+    rng = np.random.default_rng(k)
+    data = rng.integers(0, 256, (n, dim)).astype(np.float32)
+    queries = rng.integers(0, 256, (nq, dim)).astype(np.float32)
+    if kind != "bytes":
+        data, queries = data + rng.random(data.shape, dtype=np.float32), queries - rng.random(queries.shape, dtype=np.float32)
+    metric = "l2" if kind == "bytes" else kind
+    ids, dists = exact_search(torch.from_numpy(data).cuda(), torch.from_numpy(queries).cuda(), k, metric)
+    o_ids, o_d = exact.exact_search(data, queries, k, metric)
+    np.testing.assert_array_equal(ids.cpu().numpy(), o_ids)
+    tol = {"bytes": 0.0, "cosine": 0.0}.get(kind, dim * 2.0**-52)
+    np.testing.assert_allclose(dists.cpu().numpy(), o_d, rtol=tol, atol=dim * 2.0**-52 if kind == "cosine" else 0.0)
