@@ -9,7 +9,7 @@ learned stop with the shipped network when ``--stop``), autotuning off, so the s
 launches are the 3 searches in order (with the start order's launches before each when
 ``nq >= 4096``). ``exact``: the tensor-core exact k-NN (k = 100) of ``nq`` mixture queries over the
 1M x 128 mixture rows (``--image``: 60K x 784 image-like rows), ``calls`` times;
-each call launches the filter kernel twice (the prefix pass, then every row).
+each call launches the filter kernel twice (a sample of the rows, then every row).
 """
 
 from __future__ import annotations
