@@ -942,9 +942,10 @@ __device__ __forceinline__ double dist_f64_warp(const T *x, const T *qv, int dim
 // Survivors (candidates within the final threshold) of a query that rerank_topk gathers in shared
 // memory and sorts there; a query with more (many exact ties) inserts them one by one.
 __host__ __device__ constexpr int survivor_slots(int k) { return k + k / 4 + 64; }
-// Shared memory of one warp of rerank_topk: distances and ids of the results and of the survivors.
+// Shared memory of one warp of rerank_topk: distances and ids of the results and of the survivors, and a
+// queue of 64 survivors for the insertion.
 __host__ __device__ inline size_t rerank_smem(int k, bool gather) {
-    return (size_t(k + 1 + (gather ? survivor_slots(k) : 0)) * 12 + 15) & ~size_t(15);
+    return (size_t(k + 1 + (gather ? survivor_slots(k) : 0)) * 12 + 64 * 8 + 15) & ~size_t(15);
 }
 
 // One warp per query: exact float64 distances of the candidates within the final threshold,
@@ -982,6 +983,8 @@ __global__ void rerank_topk(const T *data, const T *queries, int dim, int32_t nq
     double *Sd = Ad + k + 1;                             // survivors
     int32_t *Ai = reinterpret_cast<int32_t *>(Sd + slots);
     int32_t *Si = Ai + k + 1;
+    float *Wv = reinterpret_cast<float *>(Si + slots);   // the queue
+    int32_t *Wi = reinterpret_cast<int32_t *>(Wv + 64);
     const float t = thr[q];
     const T *qv = queries + int64_t(q) * dim;
     const bool cos = metric == HNSW_B200_COSINE;
@@ -1053,11 +1056,33 @@ __global__ void rerank_topk(const T *data, const T *queries, int dim, int32_t nq
         a = min(ns, k);
         __syncwarp();
     } else {
-        for (int b0 = 0; b0 < m; b0 += 32) {
-            const int64_t at = b0 + lane < m ? region + b0 + lane : -1;  // this lane's entry
-            const float approx = at >= 0 ? cand_val[at] : INFINITY;
-            const bool has = at >= 0 && approx <= t;
-            const int32_t id = has ? cand_id[at] : -1;
+        // Survivors wait in a queue until there are 32: scored as they come, a float64 chain would run for the
+        // few of a batch of candidates (1,000 queries x 2,000 x 64 floats, cosine, k = 400: 937 -> 647 us).
+        int held = 0;
+        for (int b0 = 0; b0 < m || held > 0; b0 += 32) {
+            const bool in = b0 + lane < m;
+            const float value = in ? cand_val[region + b0 + lane] : INFINITY;
+            const uint32_t hm = __ballot_sync(0xffffffffu, in && value <= t);
+            if ((hm >> lane) & 1u) {
+                const int at = held + __popc(hm & ((1u << lane) - 1u));
+                Wv[at] = value;
+                Wi[at] = cand_id[region + b0 + lane];
+            }
+            held += __popc(hm);
+            if (held < 32 && b0 + 32 < m) continue;  // uniform
+            __syncwarp();
+            const bool has = lane < held;
+            const float approx = has ? Wv[lane] : INFINITY;
+            const int32_t id = has ? Wi[lane] : -1;
+            const bool more = 32 + lane < held;
+            const float next_v = more ? Wv[32 + lane] : 0.f;
+            const int32_t next_i = more ? Wi[32 + lane] : 0;
+            __syncwarp();
+            if (more) {
+                Wv[lane] = next_v;
+                Wi[lane] = next_i;
+            }
+            held = max(held - 32, 0);
             const bool known = has && fabsf(approx) < exact_lim;  // exact already (byte rows)
             const bool need = has && !known;
             double d = known ? double(approx) : INFINITY;
@@ -1274,6 +1299,11 @@ size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Candidate lists take at most CAND_BYTES of scratch: (query, segment) pairs x cap x 8 bytes.
 constexpr int64_t CAND_BYTES = int64_t(4) << 30;
+// and this much, whatever candidates are expected, as long as segments stay below the columns that they cover: rows
+// stored by cluster or by time fill few segments, and an overflow runs the call again. 1,000 queries x 1M x 128
+// bytes in runs of 1,000 similar rows, k = 10, 2.26 -> 1.27 ms; 1,000 x 200K x 100 floats in runs of 2,000, cosine, k =
+// 10, 1.28 -> 0.79 ms; rows in no order take the same time.
+constexpr int64_t CAND_ROOM = int64_t(2) << 30;
 constexpr int64_t MAX_CHUNK = 16384;  // queries of a batch filtered together
 // A segment of pass two is sized for SEGMENT_FACTOR times its even share of the candidates expected, for
 // thresholds looser than expected and uneven shares, and for SEGMENT_SLACK entries more: the columns it has
@@ -1301,7 +1331,8 @@ constexpr double SAMPLE_BALANCE = 75.0;
 // smallest lies beyond the k-th nearest of all rows but for about one query in 10^9, while only about
 // (k f + 6 sqrt(k f) + 8) / f rows pass it (at k = 100, f = 1/8: 330; the sample's k-th
 // smallest, which is never too low, let 830 pass). Pass two counts: where a threshold was too low after
-// all (rows in an order that the stride resonates with) the chunk runs again with the k-th smallest.
+// all (rows stored by cluster or by time, a query's near ones in a sampled tile) the chunk runs again with
+// the k-th smallest.
 int sample_rank(int64_t k, int64_t sample_tiles, int64_t tiles) {
     if (sample_tiles >= tiles) return int(k);
     const double mean = double(k) * double(sample_tiles) / double(tiles);
@@ -1387,15 +1418,18 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
     const int64_t expect2 = int64_t(rank) * tiles / sample + int64_t(k) / 2;  // candidates of a query
     int64_t QB = std::min<int64_t>(nq_all, MAX_CHUNK);  // queries per chunk
     int64_t cap = 0, slots = 0;                           // entries per segment; (query, segment) pairs
+    int64_t most = 0;  // columns of a segment of pass two
     for (;;) {
-        cap = slots = 0;
+        cap = slots = most = 0;
         const int64_t last = nq_all % QB ? nq_all % QB : QB;
         for (int64_t nqc : {QB, last}) {
             const Split g1 = geo(nqc, sample), g2 = geo(nqc, tiles);
-            const int64_t nseg2 = int64_t(g2.splits) * EPI_PER_QUARTER;
+            const int64_t nseg2 = int64_t(g2.splits) * EPI_PER_QUARTER, columns = int64_t(2 * CW) * g2.tps;
             const int64_t share = (SEGMENT_FACTOR * expect2 + nseg2 - 1) / nseg2 + SEGMENT_SLACK;
-            cap = std::max<int64_t>(cap, !block_min ? int64_t(2 * CW) * g1.tps : tile_blocks ? int64_t(tile_blocks) * g1.tps : (g1.tps + 1) / 2);
-            cap = std::max<int64_t>(cap, std::min<int64_t>(std::max(cap_min, share), int64_t(2 * CW) * g2.tps));
+            cap = std::max<int64_t>(cap, !block_min ? int64_t(2 * CW) * g1.tps
+                                         : tile_blocks ? int64_t(tile_blocks) * g1.tps : (g1.tps + 1) / 2);
+            cap = std::max<int64_t>(cap, std::min(std::max(cap_min, share), columns));
+            most = std::max(most, columns);
             slots = std::max<int64_t>(slots, nqc * std::max(g1.splits, g2.splits) * EPI_PER_QUARTER);
         }
         if (slots * cap * 8 <= CAND_BYTES || QB <= BM) break;
@@ -1421,11 +1455,16 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
     const size_t o_tau = carve(size_t(QB) * 4);
     const size_t o_cnt = carve(size_t(slots) * 4);
     const size_t o_cm = carve(size_t(QB) * 4);
-    const size_t o_cv = carve(size_t(slots) * cap * 4);
-    const size_t o_ci = carve(size_t(slots) * cap * 4);
     const size_t o_st = carve(sizeof(Stats));
     const size_t o_mx = carve(16);
-    char *B = static_cast<char *>(buf.get(off));
+    // The lists last: longer where memory allows (CAND_ROOM), else as long as they have to be.
+    const int64_t roomy = std::max(cap, std::min(most, CAND_ROOM / (8 * slots)));
+    const size_t o_cv = off;
+    auto list_bytes = [&](int64_t entries) { return al256(size_t(slots) * entries * 4); };
+    char *B = static_cast<char *>(buf.get(off + 2 * list_bytes(roomy)));
+    if (B) cap = roomy;
+    else B = static_cast<char *>(buf.get(off + 2 * list_bytes(cap)));
+    const size_t o_ci = o_cv + list_bytes(cap);
     if (!B) return fail(HNSW_B200_ENOMEM, "exact knn scratch allocation failed");
     auto *xb = reinterpret_cast<__nv_bfloat16 *>(B + o_xb);
     auto *qb = reinterpret_cast<__nv_bfloat16 *>(B + o_qb);
@@ -1487,13 +1526,13 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
     const int wpb = 4;
     if (size_t(wpb) * (k + 1) * 12 > 200 * 1024) return fail(HNSW_B200_EINVAL, "k too large for the rerank kernel");
     // Survivors are gathered where that leaves an SM two blocks of four queries (k up to about 1,000), under cosine
-    // nine (k up to about 210): a lane's divisions want many warps, which the insertion's smaller memory lets
-    // in. Time of a search with them gathered over inserted, 20K to 100K rows of 32 to 400 values, 100 to 10K
+    // eight (k up to about 220): a lane's divisions want many warps, which the insertion's smaller memory lets
+    // in. Time of a search with them gathered over inserted (before the insertion's queue), 20K to 100K rows of 32 to 400 values, 100 to 10K
     // queries: l2 and ip 0.67 to 1.14 up to k = 1,000 and 0.74 to 1.53 above, bytes 0.63 to 1.05 and 0.71 to
     // 1.31, cosine 0.58 to 0.99 up to k = 200 and 0.69 to 1.77 above. (With the products of a batch's rows laid out in
     // shared memory as well, cosine at k = 10 took the same time, and from k = 1,000 on up to 1.5 times the time
     // without.)
-    const bool gather = wpb * rerank_smem(k, true) * (cos ? 9 : 2) <= size_t(SMEM_MAX);
+    const bool gather = wpb * rerank_smem(k, true) * (cos ? 8 : 2) <= size_t(SMEM_MAX);
     const size_t rsm = wpb * rerank_smem(k, gather);
     XT(cudaFuncSetAttribute(rerank_topk<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(rsm)));
     XT(cudaMemsetAsync(st, 0, sizeof(Stats), s));

@@ -187,3 +187,48 @@ def test_results_at_every_size_of_block(kind: str, k: int) -> None:
     np.testing.assert_array_equal(ids.cpu().numpy(), o_ids)
     tol = {"bytes": 0.0, "cosine": 0.0}.get(kind, dim * 2.0**-52)
     np.testing.assert_allclose(dists.cpu().numpy(), o_d, rtol=tol, atol=dim * 2.0**-52 if kind == "cosine" else 0.0)
+
+
+def test_lists_beyond_their_room_are_collected_again() -> None:
+    """Every row at one distance of every query, and more queries than lists as long as the rows have room for: the
+    first attempt overflows, and the next ones take fewer queries at a time."""
+    import torch
+
+    from hnsw_engine_b200 import _lib
+    from hnsw_engine_b200.exact_knn import exact_search
+
+    n, nq, k = 200_000, 4_000, 7
+    lib = _lib.load()
+    with pytest.raises(_lib.HnswB200Error):
+        _lib.check(lib.hnsw_b200_pack_mask(None, None, 1, None, None))  # the thread's last failure
+    before = lib.hnsw_b200_last_error()
+    data = torch.full((n, 8), 3.0, device="cuda")
+    data[n - 5] = 4.0  # one row nearer than the rest
+    queries = torch.full((nq, 8), 6.0, device="cuda")
+    ids, dists = exact_search(data, queries, k, "l2")
+    assert lib.hnsw_b200_last_error() != before  # the overflow
+    np.testing.assert_array_equal(ids.cpu().numpy(), np.tile([n - 5, 0, 1, 2, 3, 4, 5], (nq, 1)))
+    np.testing.assert_array_equal(dists.cpu().numpy(), np.tile([32.0] + [72.0] * 6, (nq, 1)))
+
+
+def test_long_runs_fit_where_there_is_room() -> None:
+    """Rows in runs of 1,000 similar ones and 200 queries: no overflow, as lists may be longer than expected."""
+    import torch
+
+    from hnsw_engine_b200 import _lib
+    from hnsw_engine_b200.exact_knn import exact_search
+
+    rng = np.random.default_rng(3)
+    n, dim, nq, k = 150_000, 32, 200, 10
+    centres = rng.random((n // 1_000, dim)) * 128 + 30
+    data = (centres[np.sort(rng.integers(0, n // 1_000, n))] + 10 * rng.standard_normal((n, dim))).astype(np.float32)
+    queries = (centres[rng.integers(0, n // 1_000, nq)] + 10 * rng.standard_normal((nq, dim))).astype(np.float32)
+    lib = _lib.load()
+    with pytest.raises(_lib.HnswB200Error):
+        _lib.check(lib.hnsw_b200_pack_mask(None, None, 1, None, None))
+    before = lib.hnsw_b200_last_error()
+    ids, dists = exact_search(torch.from_numpy(data).cuda(), torch.from_numpy(queries).cuda(), k, "l2")
+    assert lib.hnsw_b200_last_error() == before
+    o_ids, o_d = exact.exact_search(data, queries, k, "l2")
+    np.testing.assert_array_equal(ids.cpu().numpy(), o_ids)
+    np.testing.assert_allclose(dists.cpu().numpy(), o_d, rtol=dim * 2.0**-52)
