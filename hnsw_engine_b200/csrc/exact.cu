@@ -1311,7 +1311,7 @@ constexpr int64_t MAX_CHUNK = 16384;  // queries of a batch filtered together
 // segment. With half a tile's columns of slack (32) such rows overflowed and the call ran twice: 10K
 // queries x 1M x 128 bytes in 10,000 runs of similar rows, k = 100, 8.36 -> 4.20 ms; 2,000 x 200K x 64 floats
 // in 10,000 runs, k = 10, 936 -> 480 us; rows in no order take the same time with either (3.21 ms,
-// 430 us). Longer runs still overflow (1,000 rows each: 12.4 ms).
+// 430 us).
 constexpr int64_t SEGMENT_FACTOR = 6;
 constexpr int64_t SEGMENT_SLACK = 4 * CW;
 // Byte rows use the integer filter (1) or the BF16 one (0).
