@@ -804,14 +804,17 @@ __device__ __forceinline__ int compact_list(float *v, int32_t *id, const int32_t
 constexpr int SELECT_WARPS = 8;
 // The query's list is first compacted in place (compact_list) and its length stored in
 // cand_m[q], so the radix passes and the re-rank read one dense run of entries.
-// final_pass: the list is pass two's, out_tau holds the threshold it was collected with (without the
+// step SELECT_FIRST: the list is pass one's. SELECT_TIGHTEN: it is what pass two could keep before segments
+// overflowed; the threshold becomes the k-th smallest of that where it is lower (a subset's k-th is never below
+// the set's). SELECT_FINAL: the list is pass two's, out_tau holds the threshold it was collected with (without the
 // margin), and *short_lists is set when that threshold turns out too low: fewer than k entries, or
 // a k-th smallest above it. stat_max: largest |value| the error bound is stated for (byte rows: the
-// finite final thresholds; else the margins), as float bits. longest (final pass): the longest segment count;
-// where lists overflowed the call runs again, and nothing here is worth doing.
+// finite final thresholds; else the margins), as float bits. longest (final step): the longest segment count;
+// where lists overflowed they are collected again, and nothing here is worth doing.
+enum SelectStep : int { SELECT_FIRST, SELECT_FINAL, SELECT_TIGHTEN };
 __global__ void select_kth(float *cand_val, int32_t *cand_id, const int32_t *cand_cnt, int32_t cap,
                            int32_t nseg, int32_t nq, int32_t k, const float *margin, float *out_thr,
-                           float *out_tau, int32_t *cand_m, int final_pass, int bytes,
+                           float *out_tau, int32_t *cand_m, SelectStep step, int bytes,
                            int32_t *short_lists, unsigned int *stat_max, const unsigned long long *longest) {
     __shared__ uint32_t hist_all[SELECT_WARPS][256];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -823,8 +826,8 @@ __global__ void select_kth(float *cand_val, int32_t *cand_id, const int32_t *can
                                cand_cnt + int64_t(q) * nseg, cap, nseg, lane);
     if (lane == 0) cand_m[q] = m;
     if (m < k) {
-        if (lane == 0) {
-            if (final_pass) atomicOr(short_lists, 1);
+        if (lane == 0 && step != SELECT_TIGHTEN) {
+            if (step == SELECT_FINAL) atomicOr(short_lists, 1);
             out_tau[q] = INFINITY;
             out_thr[q] = INFINITY;
         }
@@ -873,7 +876,8 @@ __global__ void select_kth(float *cand_val, int32_t *cand_id, const int32_t *can
     }
     if (lane == 0) {
         const float tau = funkey(prefix), mg = margin[q];
-        if (final_pass) {
+        if (step == SELECT_TIGHTEN && !(tau < out_tau[q])) return;
+        if (step == SELECT_FINAL) {
             if (!(tau <= out_tau[q])) atomicOr(short_lists, 1);
             const float b = bytes ? fabsf(tau + mg) : mg;
             const unsigned int bits = isfinite(b) || !bytes ? __float_as_uint(b) : 0u;
@@ -1299,11 +1303,12 @@ size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Candidate lists take at most CAND_BYTES of scratch: (query, segment) pairs x cap x 8 bytes.
 constexpr int64_t CAND_BYTES = int64_t(4) << 30;
-// and this much, whatever candidates are expected, as long as segments stay below the columns that they cover: rows
+// and this much, whatever candidates are expected, or twice as much where segments are then as long as the columns
+// that they cover (a list just too short for its rows costs most): rows
 // stored by cluster or by time fill few segments, and an overflow runs the call again. 1,000 queries x 1M x 128
 // bytes in runs of 1,000 similar rows, k = 10, 2.26 -> 1.27 ms; 1,000 x 200K x 100 floats in runs of 2,000, cosine, k =
 // 10, 1.28 -> 0.79 ms; rows in no order take the same time.
-constexpr int64_t CAND_ROOM = int64_t(2) << 30;
+constexpr int64_t CAND_ROOM = int64_t(1) << 30;
 constexpr int64_t MAX_CHUNK = 16384;  // queries of a batch filtered together
 // A segment of pass two is sized for SEGMENT_FACTOR times its even share of the candidates expected, for
 // thresholds looser than expected and uneven shares, and for SEGMENT_SLACK entries more: the columns it has
@@ -1458,7 +1463,7 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
     const size_t o_st = carve(sizeof(Stats));
     const size_t o_mx = carve(16);
     // The lists last: longer where memory allows (CAND_ROOM), else as long as they have to be.
-    const int64_t roomy = std::max(cap, std::min(most, CAND_ROOM / (8 * slots)));
+    const int64_t roomy = std::max(cap, most <= CAND_ROOM / (4 * slots) ? most : CAND_ROOM / (8 * slots));
     const size_t o_cv = off;
     auto list_bytes = [&](int64_t entries) { return al256(size_t(slots) * entries * 4); };
     char *B = static_cast<char *>(buf.get(off + 2 * list_bytes(roomy)));
@@ -1593,32 +1598,44 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
             launches++;
             return 0;
         };
+        const int sel_blocks = int((nq + SELECT_WARPS - 1) / SELECT_WARPS);
+        auto select = [&](SelectStep step, int32_t *ids, int sel_rank) {
+            const bool last = step == SELECT_FINAL;
+            select_kth<<<sel_blocks, 32 * SELECT_WARPS, 0, s>>>(
+                cv, ids, cnt, int32_t(cap), int32_t(nseg), int32_t(nq), sel_rank, mg, th, tau, cm, step, bytes,
+                last ? &st->short_lists : nullptr, last ? &st->bound : nullptr, last ? &st->longest : nullptr);
+            launches++;
+        };
         for (int pass_rank = rank;; pass_rank = k) {
             // Pass one: the sampled tiles give tau, the threshold of pass two.
             if (int rc = run_filter(sample, stride, nullptr, block_min)) return rc;
-            const int sel_blocks = int((nq + SELECT_WARPS - 1) / SELECT_WARPS);
-            select_kth<<<sel_blocks, 32 * SELECT_WARPS, 0, s>>>(
-                cv, nullptr, cnt, int32_t(cap), int32_t(nseg), int32_t(nq), pass_rank, mg, th, tau, cm, 0,
-                bytes, nullptr, nullptr, nullptr);
+            select(SELECT_FIRST, nullptr, pass_rank);
             // Pass two: every row against tau + margin; the k-th smallest candidate is the global
-            // k-th approximate distance, the final threshold.
-            if (int rc = run_filter(tiles, 1, th, false)) return rc;
-            count_stats<<<int(std::min<int64_t>(1024, (nq * nseg + 255) / 256)), 256, 0, s>>>(
-                cnt, nq * nseg, &st->longest);
-            select_kth<<<sel_blocks, 32 * SELECT_WARPS, 0, s>>>(
-                cv, ci, cnt, int32_t(cap), int32_t(nseg), int32_t(nq), k, mg, th, tau, cm, 1, bytes,
-                &st->short_lists, &st->bound, &st->longest);
-            rerank_topk<T><<<int((nq + wpb - 1) / wpb), wpb * 32, rsm, s>>>(
-                X, Q, dim, int32_t(nq), k, metric, xn, qn, cv, ci, cm, int32_t(cap), int32_t(nseg), th,
-                a->out_ids + q0 * k, a->out_dists + q0 * k, &st->filter_err, bytes ? EXACT_LIM : 0.f,
-                &st->mismatch, gather, &st->longest,
-                pass_rank == k ? nullptr : &st->short_lists);
-            XT(cudaGetLastError());
-            launches += 4;
-            XT(cudaMemcpyAsync(&hst, st, sizeof(Stats), cudaMemcpyDeviceToHost, s));
-            XT(cudaMemsetAsync(st, 0, offsetof(Stats, filter_err), s));
-            XT(cudaStreamSynchronize(s));
-            if (hst.err) return fail(HNSW_B200_ECUDA, "exact knn: a bounded wait expired in the filter kernel");
+            // k-th approximate distance, the final threshold. Where segments overflow, what they kept gives a
+            // lower tau, and the pass runs again, twice at most: a loose threshold (rows stored by cluster or by time)
+            // costs a pass and not a call with longer lists, which is left for exact ties and the like. 10K queries x
+            // 1M x 128 bytes in runs of similar rows: 10,000 rows each, k = 10, 32.4 -> 15.2 ms; 1,000, k = 100, 12.5 ->
+            // 10.8 ms; but 1,000, k = 1,000, 28.8 -> 37.7 ms, and rows drifting along a path, k = 100, 73 -> 97 ms, where
+            // the passes do not suffice. (A second one only where the first halved the longest segment: 35, 17.0, 37.6,
+            // 84 ms.)
+            for (int again = 0;; again++) {
+                if (int rc = run_filter(tiles, 1, th, false)) return rc;
+                count_stats<<<int(std::min<int64_t>(1024, (nq * nseg + 255) / 256)), 256, 0, s>>>(
+                    cnt, nq * nseg, &st->longest);
+                select(SELECT_FINAL, ci, k);
+                rerank_topk<T><<<int((nq + wpb - 1) / wpb), wpb * 32, rsm, s>>>(
+                    X, Q, dim, int32_t(nq), k, metric, xn, qn, cv, ci, cm, int32_t(cap), int32_t(nseg), th,
+                    a->out_ids + q0 * k, a->out_dists + q0 * k, &st->filter_err, bytes ? EXACT_LIM : 0.f,
+                    &st->mismatch, gather, &st->longest, pass_rank == k ? nullptr : &st->short_lists);
+                XT(cudaGetLastError());
+                launches += 2;
+                XT(cudaMemcpyAsync(&hst, st, sizeof(Stats), cudaMemcpyDeviceToHost, s));
+                XT(cudaMemsetAsync(st, 0, offsetof(Stats, filter_err), s));
+                XT(cudaStreamSynchronize(s));
+                if (hst.err) return fail(HNSW_B200_ECUDA, "exact knn: a bounded wait expired in the filter kernel");
+                if (int64_t(hst.longest) <= cap || again == 2) break;
+                select(SELECT_TIGHTEN, nullptr, k);
+            }
             if (int64_t(hst.longest) > cap) {
                 *cap_needed = int64_t(hst.longest);
                 return fail(HNSW_B200_ERETRY, "exact knn: candidate buffer overflow (" +

@@ -232,3 +232,32 @@ def test_long_runs_fit_where_there_is_room() -> None:
     o_ids, o_d = exact.exact_search(data, queries, k, "l2")
     np.testing.assert_array_equal(ids.cpu().numpy(), o_ids)
     np.testing.assert_allclose(dists.cpu().numpy(), o_d, rtol=dim * 2.0**-52)
+
+
+@pytest.mark.parametrize("as_bytes", [True, False])
+def test_a_loose_threshold_costs_a_pass_not_the_call(as_bytes: bool) -> None:
+    """Rows in runs far longer than lists have room for: what overflowing segments kept tightens the threshold, and
+    no call with longer lists is needed."""
+    import torch
+
+    from hnsw_engine_b200 import _lib
+    from hnsw_engine_b200.exact_knn import exact_search
+
+    g = torch.Generator("cuda").manual_seed(5)
+    n, dim, nq, run, k = 400_000, 24, 2_000, 20_000, 10
+    centres = torch.rand((n // run, dim), generator=g, device="cuda") * 128 + 30
+    label = torch.randint(0, n // run, (n,), generator=g, device="cuda").sort().values
+    data = centres[label] + 20 * torch.randn((n, dim), generator=g, device="cuda")
+    queries = centres[torch.randint(0, n // run, (nq,), generator=g, device="cuda")]
+    queries = queries + 20 * torch.randn((nq, dim), generator=g, device="cuda")
+    if as_bytes:
+        data, queries = data.round().clamp(0, 255), queries.round().clamp(0, 255)
+    lib = _lib.load()
+    with pytest.raises(_lib.HnswB200Error):
+        _lib.check(lib.hnsw_b200_pack_mask(None, None, 1, None, None))  # the thread's last failure
+    before = lib.hnsw_b200_last_error()
+    ids, dists = exact_search(data, queries, k, "l2")
+    assert lib.hnsw_b200_last_error() == before  # an overflow that ends the attempt would have been recorded
+    o_ids, o_d = exact.exact_search(data.cpu().numpy(), queries[:48].cpu().numpy(), k, "l2")
+    np.testing.assert_array_equal(ids[:48].cpu().numpy(), o_ids)
+    np.testing.assert_allclose(dists[:48].cpu().numpy(), o_d, rtol=0 if as_bytes else dim * 2.0**-52)
