@@ -89,8 +89,7 @@ struct FilterParams {
     int32_t stages;        // operand stages in flight
     int32_t a_resident;    // the query tile's operand is loaded once and stays (else with each stage)
     int32_t tiles_per_split;
-    int32_t tile_blocks;   // threshold pass: blocks of an epilogue thread's part of a tile: 1, 2, 4, 8 or 16 (groups
-                           // of four rows); 0: a block is the thread's part of two tiles
+    int32_t block_tiles;   // threshold pass: tiles of a block of rows (see the pass), or 0: a block is four rows
     int32_t metric;
     const float *qq;       // |q|^2 per query (l2)
     const float *xx;       // per row: |x|^2 (l2) or 0; +inf past the data rows
@@ -550,7 +549,7 @@ __global__ void __launch_bounds__(FILTER_THREADS, 1)
         E.cap = p.cap;
         E.cnt = 0;  // this thread's appends (its own segment: no atomics)
         const int c0 = part * CW, c1 = c0 + CW * EPI_PER_QUARTER;
-        typename EpiThread<I8>::V bm = 0;  // threshold pass: the current block's minimum
+        typename EpiThread<I8>::V bm[CW / 4];  // threshold pass: the current blocks' minima
         for (int lt = 0; lt < ntiles; lt++) {
             const int b = lt & 1;
             const int row0 = (t0 + lt) * p.tile_stride * BN;
@@ -569,15 +568,21 @@ __global__ void __launch_bounds__(FILTER_THREADS, 1)
             const unsigned char *xslot = xring + (lt % XSLOTS) * BN * 4;
             const int valid0 = p.row_end - row0 - c0, valid1 = p.row_end - row0 - c1;
             uint32_t r0[CW], r1[CW];
-            typename EpiThread<I8>::V mg[CW / 4], bmg[CW / 4];
+            typename EpiThread<I8>::V mg[CW / 4];
             tmem_ld(tbase + uint32_t(c0), r0);
             tmem_wait(r0);
             tmem_ld(tbase + uint32_t(c1), r1);  // in flight while the first chunk is worked on
             const auto m0 = E.minima(r0, xslot + c0 * 4, mg);
             if constexpr (BMIN) {
-                if (p.tile_blocks == 16 && qvalid) E.keep(mg, 8);
+                if (p.block_tiles == 0) {
+                    if (qvalid) E.keep(mg, CW / 4);
+                } else if ((lt & (p.block_tiles - 1)) == 0) {
 #pragma unroll
-                for (int g = 0; g < CW / 4; g++) bmg[g] = mg[g];
+                    for (int g = 0; g < CW / 4; g++) bm[g] = mg[g];
+                } else {
+#pragma unroll
+                    for (int g = 0; g < CW / 4; g++) bm[g] = min2(bm[g], mg[g]);
+                }
             }
             if (!BMIN && __any_sync(0xffffffffu, E.pass(m0)))
                 E.append(tbase + uint32_t(c0), xslot + c0 * 4, row0 + c0, valid0, mg);
@@ -591,30 +596,39 @@ __global__ void __launch_bounds__(FILTER_THREADS, 1)
                 mbar_arrive(tempty + b);
                 mbar_arrive(xempty + lt % XSLOTS);
             }
-            // Threshold pass: one value per block, its minimum. The r-th smallest of the blocks' minima is at
-            // least the r-th smallest of all the values (a subset's r-th is never below the set's), and nearly as
-            // tight where there are at least twice as many blocks (see tile_blocks at the host). Values only: the
-            // pass needs no row ids.
+            // Threshold pass: one value per block, its minimum. A block is the g-th groups of four columns of
+            // this thread's chunks of block_tiles tiles: of rows in any order as good as one of neighbouring
+            // rows, and where near rows are neighbours (rows stored by cluster or by time) they are in many
+            // blocks and not in one (10K queries x 1M x 128 bytes in runs of 1,000 similar rows, k = 100: 10.8 ->
+            // 7.6 ms; 500K x 64 in tight ones, inner product, 1,000 queries, k = 10: 1.54 -> 1.03). The r-th smallest of the blocks' minima is at least the r-th smallest of all
+            // the values (a subset's r-th is never below the set's), and nearly as tight where there are at
+            // least twice as many blocks (see the host). Values only: the pass needs no row ids.
             if constexpr (BMIN) {
-                if (p.tile_blocks == 16) {
-                    if (qvalid) E.keep(mg, 8);
+                if (p.block_tiles == 0) {
+                    if (qvalid) E.keep(mg, CW / 4);
                 } else {
 #pragma unroll
-                    for (int g = 0; g < 8; g++) bmg[g] = min2(bmg[g], mg[g]);
-                    if (p.tile_blocks <= 4) {
+                    for (int g = 0; g < CW / 4; g++) bm[g] = min2(bm[g], mg[g]);
+                    const int in = lt & (p.block_tiles - 1);
+                    if (in == p.block_tiles - 1 || lt + 1 == ntiles) {
+                        // Fewer tiles than block_tiles (the CTA's last ones): as many fewer blocks.
+                        int count = CW / 4;
+                        if (2 * (in + 1) <= p.block_tiles) {
+                            count = 4;
 #pragma unroll
-                        for (int g = 0; g < 4; g++) bmg[g] = min2(bmg[g], bmg[g + 4]);
+                            for (int g = 0; g < 4; g++) bm[g] = min2(bm[g], bm[g + 4]);
+                        }
+                        if (4 * (in + 1) <= p.block_tiles) {
+                            count = 2;
+                            bm[0] = min2(bm[0], bm[2]);
+                            bm[1] = min2(bm[1], bm[3]);
+                        }
+                        if (8 * (in + 1) <= p.block_tiles) {
+                            count = 1;
+                            bm[0] = min2(bm[0], bm[1]);
+                        }
+                        if (qvalid) E.keep(bm, count);
                     }
-                    if (p.tile_blocks <= 2) {
-                        bmg[0] = min2(bmg[0], bmg[2]);
-                        bmg[1] = min2(bmg[1], bmg[3]);
-                    }
-                    if (p.tile_blocks <= 1) bmg[0] = min2(bmg[0], bmg[1]);
-                    if (p.tile_blocks == 0) {  // the part of two tiles
-                        bmg[0] = b == 0 ? bmg[0] : min2(bm, bmg[0]);
-                        bm = bmg[0];
-                    }
-                    if (qvalid && (p.tile_blocks > 0 || b == 1 || lt + 1 == ntiles)) E.keep(bmg, max(1, p.tile_blocks));
                 }
             }
         }
@@ -1400,7 +1414,7 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
 
     // Split of a pass over `tiles` tiles for a chunk of nqc queries.
     auto geo = [&](int64_t nqc, int tiles) { return split_tiles(int((nqc + BM - 1) / BM), tiles, sms); };
-    // Pass one keeps the minimum of every block of rows (tile_blocks), or every row where the sample has fewer than
+    // Pass one keeps the minimum of every block of rows (block_tiles), or every row where the sample has fewer than
     // 4 k; pass two keeps the rows within tau + margin. Each epilogue thread appends to its own segment of the query's list: in pass one at most one entry per block
     // or its 2 CW columns of a tile; pass two's segments get SEGMENT_FACTOR times their even share of the
     // expected candidates and SEGMENT_SLACK more, and never more than the columns that they cover (an
@@ -1416,9 +1430,10 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
     // minima, and fewer blocks make a looser threshold (1,000 rows' k-th of k minima is their largest) while every
     // row kept makes pass one append, which takes ten times as long (200 queries x 700 rows, k = 10: 68 us of a
     // call's 225).
-    int tile_blocks = int64_t(sample) / 2 * EPI_PER_QUARTER >= 2 * int64_t(k) ? 0 : 1;
-    while (tile_blocks > 0 && tile_blocks < 16 && whole * EPI_PER_QUARTER * tile_blocks < 2 * int64_t(k)) tile_blocks *= 2;
-    const bool block_min = tile_blocks < 16 || sampled / 4 >= k;
+    constexpr int GROUPS = CW / 4 * EPI_PER_QUARTER;  // blocks of a query in block_tiles tiles
+    int block_tiles = 16;
+    while (block_tiles > 0 && whole / block_tiles * GROUPS < 2 * int64_t(k)) block_tiles /= 2;
+    const bool block_min = block_tiles > 0 || sampled / 4 >= k;
     const int rank = sample_rank(k, sample, tiles);
     const int64_t expect2 = int64_t(rank) * tiles / sample + int64_t(k) / 2;  // candidates of a query
     int64_t QB = std::min<int64_t>(nq_all, MAX_CHUNK);  // queries per chunk
@@ -1432,7 +1447,7 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
             const int64_t nseg2 = int64_t(g2.splits) * EPI_PER_QUARTER, columns = int64_t(2 * CW) * g2.tps;
             const int64_t share = (SEGMENT_FACTOR * expect2 + nseg2 - 1) / nseg2 + SEGMENT_SLACK;
             cap = std::max<int64_t>(cap, !block_min ? int64_t(2 * CW) * g1.tps
-                                         : tile_blocks ? int64_t(tile_blocks) * g1.tps : (g1.tps + 1) / 2);
+                                         : block_tiles ? CW / 4 * int64_t((g1.tps + block_tiles - 1) / block_tiles) : int64_t(2 * CW / 4) * g1.tps);
             cap = std::max<int64_t>(cap, std::min(std::max(cap_min, share), columns));
             most = std::max(most, columns);
             slots = std::max<int64_t>(slots, nqc * std::max(g1.splits, g2.splits) * EPI_PER_QUARTER);
@@ -1573,7 +1588,7 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
             fp.stages = nstages;
             fp.a_resident = resident ? 1 : 0;
             fp.tiles_per_split = gg.tps;
-            fp.tile_blocks = tile_blocks;
+            fp.block_tiles = block_tiles;
             fp.metric = metric;
             fp.qq = qq;
             fp.xx = xx;
@@ -1614,10 +1629,9 @@ int exact_knn_typed(const hnsw_b200_exact_args_t *a, cudaStream_t s, int64_t cap
             // k-th approximate distance, the final threshold. Where segments overflow, what they kept gives a
             // lower tau, and the pass runs again, twice at most: a loose threshold (rows stored by cluster or by time)
             // costs a pass and not a call with longer lists, which is left for exact ties and the like. 10K queries x
-            // 1M x 128 bytes in runs of similar rows: 10,000 rows each, k = 10, 32.4 -> 15.2 ms; 1,000, k = 100, 12.5 ->
-            // 10.8 ms; but 1,000, k = 1,000, 28.8 -> 37.7 ms, and rows drifting along a path, k = 100, 73 -> 97 ms, where
-            // the passes do not suffice. (A second one only where the first halved the longest segment: 35, 17.0, 37.6,
-            // 84 ms.)
+            // 1M x 128 bytes in runs of similar rows (with blocks of neighbouring rows): 10,000 rows each, k = 10, 32.4 ->
+            // 15.2 ms; 1,000, k = 100, 12.5 -> 10.8 ms; but 1,000, k = 1,000, 28.8 -> 37.7 ms, where the passes do not
+            // suffice. (A second one only where the first halved the longest segment: 35, 17.0, 37.6 ms.)
             for (int again = 0;; again++) {
                 if (int rc = run_filter(tiles, 1, th, false)) return rc;
                 count_stats<<<int(std::min<int64_t>(1024, (nq * nseg + 255) / 256)), 256, 0, s>>>(

@@ -166,17 +166,18 @@ def test_lists_that_overflow_are_collected_again(as_bytes: bool, run: int, k: in
     np.testing.assert_allclose(dists.cpu().numpy(), o_d, rtol=0 if as_bytes else dim * 2.0**-52)
 
 
-# k over the blocks of the threshold pass (two tiles, a tile's part, its halves to sixteenths, every row) and over the
-# sizes at which survivors are gathered (cosine about 210, else about 1,050).
-@pytest.mark.parametrize("k", [1, 10, 20, 50, 100, 200, 213, 400, 600, 1_040, 1_060])
+# k and n over the blocks of the threshold pass (groups of four columns over 16 tiles to one, single groups, every row)
+# and k over the sizes at which survivors are gathered (cosine about 220, else about 1,040).
+@pytest.mark.parametrize("n,k", [(2_000, k) for k in (1, 10, 20, 50, 100, 200, 213, 222, 400, 600, 1_030, 1_060)]
+                         + [(30_011, k) for k in (1, 7, 70, 150, 400)])
 @pytest.mark.parametrize("kind", ["bytes", "l2", "ip", "cosine"])
-def test_results_at_every_size_of_block(kind: str, k: int) -> None:
+def test_results_at_every_size_of_block(kind: str, n: int, k: int) -> None:
     import torch
 
     from hnsw_engine_b200.exact_knn import exact_search
 
-    n, dim, nq = 2_000, 24, 70
-    rng = np.random.default_rng(k)
+    dim, nq = 24, 70
+    rng = np.random.default_rng(n + k)
     data = rng.integers(0, 256, (n, dim)).astype(np.float32)
     queries = rng.integers(0, 256, (nq, dim)).astype(np.float32)
     if kind != "bytes":
